@@ -2,15 +2,21 @@
 //
 //   a_t = h_{t-1} W + k_t (x) v_t ;  h_t = f_t h_{t-1} + (1 - f_t) tanh(a_t) ;  y_t = q_t . h_t
 //
-// One CTA per (batch, head).  The state h [KD x 16] lives in registers for the whole sequence:
-// thread (k, quad) owns h[k, 4*quad .. 4*quad+3]; the four threads of a row are adjacent lanes and
-// exchange their quads with shuffles for the 16x16 state transition.  Inputs are staged through
-// shared memory in blocks of 32 time steps (next block prefetched into registers while the
-// current one runs); y partial sums are reduced over k once per block.  The forward pass can
-// write the state history (fp32) that the backward pass replays in reverse; the backward pass
-// recomputes tanh(a_t) from h_{t-1}, keeps dh in registers, accumulates dW per thread over time
-// and reduces it once at the end.  q and k gradients are produced per head (the caller sums the
-// head axis when q/k are shared by all heads).
+// One CTA per (batch, head), one warp per 16 rows of the state h [KD x 16], which stays in registers for the whole sequence
+// in the accumulator layout of mma.m16n8k16 (lane (g, t): rows g and g + 8, columns 2t, 2t + 1 of each 8-column half).  That
+// layout is also the A operand of the next step's product with W, so a step exchanges nothing between lanes.  The products
+// keep fp32 operands: W is bf16 as given, and the fp32 factor is the sum of three bf16 parts (8 + 8 + 8 mantissa bits), each
+// multiplied exactly and added in fp32.
+//
+// What bounds it: the chain of dependent steps, not arithmetic or memory (one warp per scheduler; 4096 steps).  With four
+// threads per row, 12 shuffles and 64 dependent multiply-adds a step and the state history fetched one step ahead, the
+// backward took 1.23 us and the forward 0.29 us a step at batch 2, 51 heads; now 0.49 and 0.26 (the history is requested four
+// steps ahead, and a warp issues 378 instructions a backward step).
+// Only dh_{t-1} = f_t dh_t + da_t W^T is on the backward's chain; the replay of tanh(a_t) and all other gradients hang off it.
+//
+// Inputs are staged through shared memory in blocks of 16 steps (the next block is loaded into registers while the current
+// one runs, one block barrier per 16 steps).  The forward writes the state history (fp32) that the backward replays in
+// reverse.  q and k gradients are produced per head (the caller sums the head axis when q / k are shared by all heads).
 // The reference runs this recurrence as Triton kernels with 64-token checkpoints
 // (cppmega/megatron/m2rnn_triton.py:243-415 forward, :662-758 backward).
 #include "common.cuh"
@@ -18,8 +24,7 @@
 namespace cm {
 
 constexpr int VD = 16;       // value head dim (fixed)
-constexpr int TB = 32;       // time steps per staging block (forward)
-constexpr int TBB = 16;      // backward (more staged arrays)
+constexpr int TB = 16;       // time steps per staging block
 
 __device__ __forceinline__ float fast_tanh(float x) {
   float y;
@@ -27,392 +32,439 @@ __device__ __forceinline__ float fast_tanh(float x) {
   return y;
 }
 
-// Forward.  One CTA owns RS = min(KD, 16) state rows of one (batch, head): 4 * RS threads, thread (row, quad) holds
-// h[row, 4 quad .. 4 quad + 3].  The 16 x 16 transition matrix sits in registers, arranged per thread in the order in
-// which the row's other three quads arrive by shuffle ("rotation d" brings quad (quad + d) % 4), so a step costs
-// 12 shuffles for the matvec and 4 for the reduction of y over the rows of a warp.  With KD > 16 a head is split
-// over KD / 16 CTAs; each writes an fp32 partial y and a small kernel adds the parts.
+// c (two 16 x 8 accumulators) = hi + mid + lo, each part as the A fragment of a 16 x 16 bf16 operand
+struct Split3 {
+  uint32_t hi[4], mid[4], lo[4];
+};
+__device__ __forceinline__ float bf_lo(uint32_t p) { return __uint_as_float(p << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t p) { return __uint_as_float(p & 0xffff0000u); }
+__device__ __forceinline__ void split3(const float (&c)[8], Split3& s) {
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    float x = c[2 * p], y = c[2 * p + 1];
+    s.hi[p] = pack_bf16(x, y);
+    x -= bf_lo(s.hi[p]); y -= bf_hi(s.hi[p]);
+    s.mid[p] = pack_bf16(x, y);
+    x -= bf_lo(s.mid[p]); y -= bf_hi(s.mid[p]);
+    s.lo[p] = pack_bf16(x, y);
+  }
+}
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// out[0..3] | out[4..7] = x M for the 16 x 16 bf16 matrix M held as B fragments
+__device__ __forceinline__ void times16(float (&out)[8], const Split3& x, const uint32_t (&m)[2][2]) {
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
+    mma16816(a, x.lo, m[n]);
+    mma16816(b, x.hi, m[n]);
+    mma16816(a, x.mid, m[n]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[n * 4 + i] = a[i] + b[i];
+  }
+}
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+// Sum of x[0..3] over the 8 lanes with equal (lane & 3); lane returns the sum of element 2 * bit4 + bit3 (bit2 is redundant).
+__device__ __forceinline__ float reduce_rows4(const float (&x)[4], int lane) {
+  const bool u4 = lane & 16, u3 = lane & 8;
+  const float a0 = (u4 ? x[2] : x[0]) + __shfl_xor_sync(0xffffffffu, u4 ? x[0] : x[2], 16);
+  const float a1 = (u4 ? x[3] : x[1]) + __shfl_xor_sync(0xffffffffu, u4 ? x[1] : x[3], 16);
+  float r = (u3 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, u3 ? a0 : a1, 8);
+  return r + __shfl_xor_sync(0xffffffffu, r, 4);
+}
+// column (0..15) of the element that reduce_rows4 leaves in this lane, for x = columns {2t, 2t + 1, 8 + 2t, 9 + 2t}
+__device__ __forceinline__ int reduced_col(int lane) { return 2 * (lane & 3) + ((lane >> 3) & 1) + ((lane & 16) ? 8 : 0); }
+
+// 8 consecutive bf16; `vec`: the address is 16-byte aligned
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, bool vec) {
+  if (vec) return *reinterpret_cast<const uint4*>(p);
+  const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+  uint4 r;
+  r.x = u[0] | (uint32_t(u[1]) << 16); r.y = u[2] | (uint32_t(u[3]) << 16);
+  r.z = u[4] | (uint32_t(u[5]) << 16); r.w = u[6] | (uint32_t(u[7]) << 16);
+  return r;
+}
+__device__ __forceinline__ void spread8(float* dst, uint4 v) {
+  reinterpret_cast<float4*>(dst)[0] = make_float4(bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y));
+  reinterpret_cast<float4*>(dst)[1] = make_float4(bf_lo(v.z), bf_hi(v.z), bf_lo(v.w), bf_hi(v.w));
+}
+
+// One block of inputs: TB steps of q, k (this head's or the shared one), v, dy and f
+template <int KD, bool BWD>
+struct Stage {
+  float q[TB][KD], k[TB][KD], v[TB][VD], g[BWD ? TB : 1][VD], f[TB];
+};
+
+template <int KD, bool BWD>
+struct Loader {
+  static constexpr int NT = KD * 2;            // threads: one 8-wide vector of q and of k each per block
+  const __nv_bfloat16 *q, *k, *v, *g;
+  const float* f;
+  size_t q_step, k_step, v_step, f_step;
+  int S;
+  bool vec;
+  uint4 rq, rk, rv, rg;
+  float rf;
+  __device__ __forceinline__ void fetch(int t0, int tid) {
+    const int t = tid / (KD / 8), c = (tid % (KD / 8)) * 8;
+    const bool in = t0 + t < S;
+    rq = in ? load8(q + (size_t)(t0 + t) * q_step + c, vec) : make_uint4(0, 0, 0, 0);
+    rk = in ? load8(k + (size_t)(t0 + t) * k_step + c, vec) : make_uint4(0, 0, 0, 0);
+    if (tid < 2 * TB) {
+      const int tv = tid >> 1, cv = (tid & 1) * 8;
+      const bool inv = t0 + tv < S;
+      rv = inv ? load8(v + (size_t)(t0 + tv) * v_step + cv, vec) : make_uint4(0, 0, 0, 0);
+      if (BWD) rg = inv ? load8(g + (size_t)(t0 + tv) * v_step + cv, vec) : make_uint4(0, 0, 0, 0);
+      if (tid < TB) rf = t0 + tid < S ? f[(size_t)(t0 + tid) * f_step] : 1.f;
+    }
+  }
+  __device__ __forceinline__ void commit(Stage<KD, BWD>& s, int tid) const {
+    const int t = tid / (KD / 8), c = (tid % (KD / 8)) * 8;
+    spread8(&s.q[t][c], rq);
+    spread8(&s.k[t][c], rk);
+    if (tid < 2 * TB) {
+      spread8(&s.v[tid >> 1][(tid & 1) * 8], rv);
+      if (BWD) spread8(&s.g[tid >> 1][(tid & 1) * 8], rg);
+      if (tid < TB) s.f[tid] = rf;
+    }
+  }
+};
+
+// B fragments of W (out[v] = sum_u x[u] W[u][v]) or of its transpose (out[u] = sum_v x[v] W[u][v])
+__device__ __forceinline__ void load_matrix(uint32_t (&m)[2][2], const __nv_bfloat16* w, int lane, bool transposed) {
+  const int g = lane >> 2, t = lane & 3;
+  const unsigned short* u = reinterpret_cast<const unsigned short*>(w);
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int kk = h * 8 + 2 * t, nn = n * 8 + g;
+      const unsigned short a = transposed ? u[nn * VD + kk] : u[kk * VD + nn];
+      const unsigned short b = transposed ? u[nn * VD + kk + 1] : u[(kk + 1) * VD + nn];
+      m[n][h] = a | (uint32_t(b) << 16);
+    }
+}
+
 template <int KD>
-struct M2Split {
-  static constexpr int RS = KD < 16 ? KD : 16;     // 16 rows = 64 threads: B*H*KD/16 CTAs balance over the SMs
-  static constexpr int SPLITS = KD / RS;
-  static constexpr int NT = RS * 4;
+__global__ void __launch_bounds__(KD * 2) m2rnn_fwd_kernel(
+    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
+    const __nv_bfloat16* __restrict__ W, const float* __restrict__ f, __nv_bfloat16* __restrict__ y, float* __restrict__ hist,
+    float* __restrict__ h_last, int S, int H, int Hq, int Hk, bool vec) {
+  constexpr int NT = KD * 2, NW = KD / 16;
+  __shared__ __align__(16) Stage<KD, false> stage[2];
+  __shared__ float ypart[2][TB][NW][VD];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  const int b = blockIdx.x / H, h = blockIdx.x % H;
+  const int r0 = warp * 16 + g;                  // state rows r0 and r0 + 8
+  Loader<KD, false> in;
+  in.q = q + ((size_t)b * S * Hq + (Hq == 1 ? 0 : h)) * KD;
+  in.k = k + ((size_t)b * S * Hk + (Hk == 1 ? 0 : h)) * KD;
+  in.v = v + ((size_t)b * S * H + h) * VD;
+  in.g = nullptr;
+  in.f = f + (size_t)b * S * H + h;
+  in.q_step = (size_t)Hq * KD; in.k_step = (size_t)Hk * KD; in.v_step = (size_t)H * VD; in.f_step = H;
+  in.S = S; in.vec = vec;
+  uint32_t w[2][2];
+  load_matrix(w, W + (size_t)h * VD * VD, lane, false);
+  float hs[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) hs[i] = 0.f;
+  float* hrow = hist ? hist + ((size_t)blockIdx.x * S * KD + r0) * VD + 2 * t4 : nullptr;
+  const int col = reduced_col(lane);
+  in.fetch(0, tid);
+  in.commit(stage[0], tid);
+  auto write_y = [&](int blk) {                  // sum of the warps' parts of block `blk`
+    const int t0 = blk * TB, nt = min(TB, S - t0);
+    for (int e = tid; e < nt * VD; e += NT) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) s += ypart[blk & 1][e / VD][i][e % VD];
+      y[((size_t)(b * S + t0 + e / VD) * H + h) * VD + e % VD] = __float2bfloat16(s);
+    }
+  };
+  const int nblocks = (S + TB - 1) / TB;
+  for (int blk = 0; blk < nblocks; ++blk) {
+    __syncthreads();                              // inputs of this block and y parts of the previous one are complete
+    const Stage<KD, false>& st = stage[blk & 1];
+    if (blk + 1 < nblocks) in.fetch((blk + 1) * TB, tid);
+    if (blk > 0) write_y(blk - 1);
+    const int nt = min(TB, S - blk * TB);
+#pragma unroll 2
+    for (int t = 0; t < nt; ++t) {
+      const float k0 = st.k[t][r0], k1 = st.k[t][r0 + 8], q0 = st.q[t][r0], q1 = st.q[t][r0 + 8], ft = st.f[t];
+      const float2 va = *reinterpret_cast<const float2*>(&st.v[t][2 * t4]), vb = *reinterpret_cast<const float2*>(&st.v[t][8 + 2 * t4]);
+      const float vv[4] = {va.x, va.y, vb.x, vb.y};
+      Split3 s;
+      split3(hs, s);
+      float a[8];
+      times16(a, s, w);
+      float yp[4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int c = (i >> 2) * 2 + (i & 1);      // column slot of element i; elements 2, 3, 6, 7 are row r0 + 8
+        const float x = fmaf((i & 2) ? k1 : k0, vv[c], a[i]);
+        hs[i] = fmaf(ft, hs[i], (1.f - ft) * fast_tanh(x));
+      }
+      if (hist) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<float2*>(hrow + ((i & 1) ? 8 * VD : 0) + (i >> 1) * 8) = make_float2(hs[2 * i], hs[2 * i + 1]);
+        hrow += (size_t)KD * VD;
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int i = (c >> 1) * 4 + (c & 1);
+        yp[c] = fmaf(q1, hs[i + 2], q0 * hs[i]);
+      }
+      const float r = reduce_rows4(yp, lane);
+      if ((lane & 4) == 0) ypart[blk & 1][t][warp][col] = r;
+    }
+    if (blk + 1 < nblocks) in.commit(stage[(blk + 1) & 1], tid);     // its last readers passed the barrier above
+  }
+  __syncthreads();
+  write_y(nblocks - 1);
+  if (h_last) {
+    float* o = h_last + ((size_t)blockIdx.x * KD + r0) * VD + 2 * t4;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<float2*>(o + ((i & 1) ? 8 * VD : 0) + (i >> 1) * 8) = make_float2(hs[2 * i], hs[2 * i + 1]);
+  }
+}
+
+template <int KD>
+struct BwdShared {
+  Stage<KD, true> stage[2];
+  float dq[2][TB][KD], dk[2][TB][KD];
+  float dv[2][TB][KD / 16][VD];
+  float df[2][TB][KD * 2 + 8];                  // one partial per lane; rows 8 banks apart
+  float dw[VD][VD];
 };
 
 template <int KD>
-__global__ void __launch_bounds__(M2Split<KD>::NT) m2rnn_fwd_kernel(
-    const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
-    const __nv_bfloat16* __restrict__ W, const float* __restrict__ f, __nv_bfloat16* __restrict__ y, float* __restrict__ y_part,
-    float* __restrict__ hist, float* __restrict__ h_last, int B, int S, int H, int Hq, int Hk) {
-  constexpr int RS = M2Split<KD>::RS, SPLITS = M2Split<KD>::SPLITS, NT = M2Split<KD>::NT;
-  constexpr int NW = NT / 32;
-  constexpr int QPT = TB * RS / NT;     // staged q (and k) elements per thread = 8
-  constexpr int VPT = (TB * VD + NT - 1) / NT;
-  __shared__ float qs[TB][RS], ks[TB][RS], fs[TB];
-  __shared__ __align__(16) float vs[TB][VD];
-  __shared__ float ypart[TB][NW][VD];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int lrow = tid >> 2, quad = tid & 3;
-  const int sp = blockIdx.x % SPLITS;
-  const int bh = blockIdx.x / SPLITS;
-  const int b = bh / H, h = bh % H;
-  const int row = sp * RS + lrow;
-  const int hq = Hq == 1 ? 0 : h, hk = Hk == 1 ? 0 : h;
-  // wrot[d][u][c] = W[4 * ((quad + d) % 4) + u][4 * quad + c]
-  float wrot[4][4][4];
-#pragma unroll
-  for (int d = 0; d < 4; ++d)
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        wrot[d][u][c] = __bfloat162float(W[(size_t)h * VD * VD + (4 * ((quad + d) & 3) + u) * VD + 4 * quad + c]);
-  float hreg[4] = {0.f, 0.f, 0.f, 0.f};
-  float pq[QPT], pk[QPT], pv[VPT], pf = 0.f;
-
-  auto prefetch = [&](int t0) {
-#pragma unroll
-    for (int i = 0; i < QPT; ++i) {
-      const int e = tid + i * NT, t = e / RS, c = e % RS;
-      const bool ok = t0 + t < S;
-      pq[i] = ok ? __bfloat162float(q[((size_t)(b * S + t0 + t) * Hq + hq) * KD + sp * RS + c]) : 0.f;
-      pk[i] = ok ? __bfloat162float(k[((size_t)(b * S + t0 + t) * Hk + hk) * KD + sp * RS + c]) : 0.f;
-    }
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int e = tid + i * NT;
-      const int t = e / VD, c = e % VD;
-      pv[i] = (e < TB * VD && t0 + t < S) ? __bfloat162float(v[((size_t)(b * S + t0 + t) * H + h) * VD + c]) : 0.f;
-    }
-    if (tid < TB) pf = (t0 + tid < S) ? f[(size_t)(b * S + t0 + tid) * H + h] : 1.f;
-  };
-  auto commit = [&]() {
-#pragma unroll
-    for (int i = 0; i < QPT; ++i) {
-      const int e = tid + i * NT;
-      qs[e / RS][e % RS] = pq[i];
-      ks[e / RS][e % RS] = pk[i];
-    }
-#pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int e = tid + i * NT;
-      if (e < TB * VD) vs[e / VD][e % VD] = pv[i];
-    }
-    if (tid < TB) fs[tid] = pf;
-  };
-
-  prefetch(0);
-  commit();
-  __syncthreads();
-  const int src_base = lane & ~3;
-  for (int t0 = 0; t0 < S; t0 += TB) {
-    if (t0 + TB < S) prefetch(t0 + TB);
-    const int nt = min(TB, S - t0);
-    for (int t = 0; t < nt; ++t) {
-      const float kt = ks[t][lrow], qt = qs[t][lrow], ft = fs[t];
-      const float4 vq = *reinterpret_cast<const float4*>(&vs[t][quad * 4]);
-      float a[4] = {kt * vq.x, kt * vq.y, kt * vq.z, kt * vq.w};
-#pragma unroll
-      for (int d = 0; d < 4; ++d) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float hv = d == 0 ? hreg[u] : __shfl_sync(0xffffffffu, hreg[u], src_base | ((quad + d) & 3));
-#pragma unroll
-          for (int c = 0; c < 4; ++c) a[c] = fmaf(hv, wrot[d][u][c], a[c]);
-        }
-      }
-      float yp[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        hreg[c] = ft * hreg[c] + (1.f - ft) * fast_tanh(a[c]);
-        yp[c] = qt * hreg[c];
-      }
-      if (hist) {
-        float4 o = make_float4(hreg[0], hreg[1], hreg[2], hreg[3]);
-        *reinterpret_cast<float4*>(hist + (((size_t)(b * H + h) * S + t0 + t) * KD + row) * VD + quad * 4) = o;
-      }
-      // sum over the 8 rows of this warp (lanes that differ in bits 2..4): 4 shuffles, halving the values kept
-      {
-        const bool u4 = lane & 16, u3 = lane & 8;
-        const float k0 = u4 ? yp[2] : yp[0], k1 = u4 ? yp[3] : yp[1];
-        const float s0 = u4 ? yp[0] : yp[2], s1 = u4 ? yp[1] : yp[3];
-        const float a0 = k0 + __shfl_xor_sync(0xffffffffu, s0, 16);
-        const float a1 = k1 + __shfl_xor_sync(0xffffffffu, s1, 16);
-        const float kk = u3 ? a1 : a0, ss = u3 ? a0 : a1;
-        float r = kk + __shfl_xor_sync(0xffffffffu, ss, 8);
-        r += __shfl_xor_sync(0xffffffffu, r, 4);
-        if ((lane & 4) == 0) ypart[t][warp][quad * 4 + (u4 ? 2 : 0) + (u3 ? 1 : 0)] = r;
-      }
-    }
-    __syncthreads();
-    for (int e = tid; e < nt * VD; e += NT) {
-      const int t = e / VD, c = e % VD;
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < NW; ++w) s += ypart[t][w][c];
-      const size_t o = ((size_t)(b * S + t0 + t) * H + h) * VD + c;
-      if (SPLITS == 1) y[o] = __float2bfloat16(s);
-      else y_part[(size_t)sp * B * S * H * VD + o] = s;
-    }
-    if (t0 + TB < S) commit();
-    __syncthreads();
-  }
-  if (h_last) {
-    float4 o = make_float4(hreg[0], hreg[1], hreg[2], hreg[3]);
-    *reinterpret_cast<float4*>(h_last + ((size_t)(b * H + h) * KD + row) * VD + quad * 4) = o;
-  }
-}
-
-__global__ void __launch_bounds__(256) m2rnn_sum_parts_kernel(const float* __restrict__ parts, __nv_bfloat16* __restrict__ y, int nparts,
-                                                              long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int p = 0; p < nparts; ++p) s += parts[(size_t)p * n + i];
-    y[i] = __float2bfloat16(s);
-  }
-}
-
-// Backward.  A CTA owns RS state rows of one (batch, head) (thread = (row, quad), W and W^T in shared memory); with
-// KD = 64 a head is split over two CTAs of 32 rows so that all CTAs are resident at once, and dv / df / dW, which sum
-// over the rows of a head, are accumulated with atomics into zeroed outputs.
-// The state history is walked backwards with rolling registers: the row h_{t-1} needed by a step was requested one
-// step earlier and h_t (own quad) is a slice of the row used by the previous step, so each step issues one row load
-// whose latency hides behind the arithmetic.
-template <int KD, int RS>
-__global__ void __launch_bounds__(RS * 4) m2rnn_bwd_kernel(
+__global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
     const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
     const __nv_bfloat16* __restrict__ W, const float* __restrict__ f, const float* __restrict__ hist,
     const __nv_bfloat16* __restrict__ dy, float* __restrict__ dq_h, float* __restrict__ dk_h,
-    float* __restrict__ dv, float* __restrict__ df, float* __restrict__ dW, int S, int H, int Hq, int Hk) {
-  constexpr int NT = RS * 4;
-  constexpr int SPLITS = KD / RS;
-  constexpr int NW = NT / 32;
-  constexpr int QPT = TBB * RS / NT;
-  __shared__ float Ws[VD][VD];          // W[u][v]
-  __shared__ float Wt[VD][VD];          // W^T: Wt[v][u]
-  __shared__ float qs[TBB][RS], ks[TBB][RS], vs[TBB][VD], gs[TBB][VD], fs[TBB];
-  __shared__ float dqs[TBB][RS], dks[TBB][RS], dvpart[TBB][NW][VD], dfpart[TBB][NW];
-  __shared__ float dWs[VD][VD];
+    float* __restrict__ dv, float* __restrict__ df, float* __restrict__ dW, int S, int H, int Hq, int Hk, bool vec) {
+  constexpr int NT = KD * 2, NW = KD / 16;
+  constexpr int AHEAD = 4;                       // steps between the request of a state and its use
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  BwdShared<KD>& sh = *reinterpret_cast<BwdShared<KD>*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int lrow = tid >> 2, quad = tid & 3;
-  const int sp = blockIdx.x % SPLITS;
-  const int bh = blockIdx.x / SPLITS;
-  const int b = bh / H, h = bh % H;
-  const int row = sp * RS + lrow;
-  const int hq = Hq == 1 ? 0 : h, hk = Hk == 1 ? 0 : h;
-  for (int i = tid; i < VD * VD; i += NT) {
-    const float w = __bfloat162float(W[(size_t)h * VD * VD + i]);
-    Ws[i / VD][i % VD] = w;
-    Wt[i % VD][i / VD] = w;
-    dWs[i / VD][i % VD] = 0.f;
-  }
-  float dh[4] = {0.f, 0.f, 0.f, 0.f};
-  float P[4][VD];
+  const int g = lane >> 2, t4 = lane & 3;
+  const int b = blockIdx.x / H, h = blockIdx.x % H;
+  const int r0 = warp * 16 + g;
+  Loader<KD, true> in;
+  in.q = q + ((size_t)b * S * Hq + (Hq == 1 ? 0 : h)) * KD;
+  in.k = k + ((size_t)b * S * Hk + (Hk == 1 ? 0 : h)) * KD;
+  in.v = v + ((size_t)b * S * H + h) * VD;
+  in.g = dy + ((size_t)b * S * H + h) * VD;
+  in.f = f + (size_t)b * S * H + h;
+  in.q_step = (size_t)Hq * KD; in.k_step = (size_t)Hk * KD; in.v_step = (size_t)H * VD; in.f_step = H;
+  in.S = S; in.vec = vec;
+  uint32_t w[2][2], wt[2][2];
+  load_matrix(w, W + (size_t)h * VD * VD, lane, false);
+  load_matrix(wt, W + (size_t)h * VD * VD, lane, true);
+  for (int i = tid; i < VD * VD; i += NT) (&sh.dw[0][0])[i] = 0.f;
+  const float* hbase = hist + ((size_t)blockIdx.x * S * KD + r0) * VD + 2 * t4;
+  auto load_state = [&](float (&x)[8], int t) {   // h_t, zero before the first step and (never used) past the last
 #pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int j = 0; j < VD; ++j) P[c][j] = 0.f;
-  const float* hbase = hist + (size_t)(b * H + h) * S * KD * VD;
-  __syncthreads();
-
-  // rolling history registers: row h_{S-2} and own quad of h_{S-1}
-  float4 rowbuf[4], quadbuf;
-  quadbuf = *reinterpret_cast<const float4*>(hbase + ((size_t)(S - 1) * KD + row) * VD + quad * 4);
-  if (S > 1) {
-    const float4* hp = reinterpret_cast<const float4*>(hbase + ((size_t)(S - 2) * KD + row) * VD);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) rowbuf[j] = hp[j];
-  } else {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) rowbuf[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  const int nblocks = (S + TBB - 1) / TBB;
-  for (int blk = nblocks - 1; blk >= 0; --blk) {
-    const int t0 = blk * TBB;
-    const int nt = min(TBB, S - t0);
-    // stage this block's inputs
-#pragma unroll
-    for (int i = 0; i < QPT; ++i) {
-      const int e = tid + i * NT, t = e / RS, c = e % RS;
-      const bool ok = t < nt;
-      qs[t][c] = ok ? __bfloat162float(q[((size_t)(b * S + t0 + t) * Hq + hq) * KD + sp * RS + c]) : 0.f;
-      ks[t][c] = ok ? __bfloat162float(k[((size_t)(b * S + t0 + t) * Hk + hk) * KD + sp * RS + c]) : 0.f;
+    for (int i = 0; i < 4; ++i) {
+      float2 p = make_float2(0.f, 0.f);
+      if (t >= 0 && t < S) p = *reinterpret_cast<const float2*>(hbase + (size_t)t * KD * VD + ((i & 1) ? 8 * VD : 0) + (i >> 1) * 8);
+      x[2 * i] = p.x; x[2 * i + 1] = p.y;
     }
-    for (int e = tid; e < TBB * VD; e += NT) {
-      const int t = e / VD, c = e % VD;
-      const bool ok = t < nt;
-      vs[t][c] = ok ? __bfloat162float(v[((size_t)(b * S + t0 + t) * H + h) * VD + c]) : 0.f;
-      gs[t][c] = ok ? __bfloat162float(dy[((size_t)(b * S + t0 + t) * H + h) * VD + c]) : 0.f;
-    }
-    if (tid < TBB) fs[tid] = (tid < nt) ? f[(size_t)(b * S + t0 + tid) * H + h] : 1.f;
-    __syncthreads();
-    for (int t = nt - 1; t >= 0; --t) {
-      const int tg = t0 + t;
-      // h_{t-1} (full row) was prefetched one step ago and h_t (own quad) is a slice of the row used then; the row
-      // for the next step (h_{t-2}) is requested now so that its latency hides behind this step's arithmetic
-      float hprev[VD];
+  };
+  const int nblocks = (S + TB - 1) / TB;
+  float hcur[8], ring[AHEAD][8], dh[8], dw_sum[2][4];
+  load_state(hcur, S - 1);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        hprev[j * 4 + 0] = rowbuf[j].x; hprev[j * 4 + 1] = rowbuf[j].y; hprev[j * 4 + 2] = rowbuf[j].z; hprev[j * 4 + 3] = rowbuf[j].w;
-      }
-      const float hcur[4] = {quadbuf.x, quadbuf.y, quadbuf.z, quadbuf.w};
-      if (tg > 1) {
-        const float4* hp = reinterpret_cast<const float4*>(hbase + ((size_t)(tg - 2) * KD + row) * VD);
+  for (int i = 0; i < AHEAD; ++i) load_state(ring[AHEAD - 1 - i], nblocks * TB - 2 - i);     // slot of step s: s % AHEAD, holds h_{s-1}
 #pragma unroll
-        for (int j = 0; j < 4; ++j) rowbuf[j] = hp[j];
-      } else {
+  for (int i = 0; i < 8; ++i) dh[i] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) rowbuf[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      const float kt = ks[t][lrow], qt = qs[t][lrow], ft = fs[t];
-      // dh_t += q_t (x) dy_t ; dq_t = h_t . dy_t
-      float dqp = 0.f;
+  for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float g = gs[t][quad * 4 + c];
-        dh[c] += qt * g;
-        dqp += hcur[c] * g;
-      }
-      dqp += __shfl_xor_sync(0xffffffffu, dqp, 1);
-      dqp += __shfl_xor_sync(0xffffffffu, dqp, 2);
-      if (quad == 0) dqs[t][lrow] = dqp;
-      // recompute tanh(a_t) for own columns
-      float a[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) a[c] = kt * vs[t][quad * 4 + c];
-#pragma unroll
-      for (int u = 0; u < VD; ++u) {
-        const float4 w = *reinterpret_cast<const float4*>(&Ws[u][quad * 4]);
-        a[0] += hprev[u] * w.x; a[1] += hprev[u] * w.y; a[2] += hprev[u] * w.z; a[3] += hprev[u] * w.w;
-      }
-      float hown[4];                     // h_{t-1}[k, own quad], selected without dynamic indexing
-#pragma unroll
-      for (int c = 0; c < 4; ++c)
-        hown[c] = quad == 0 ? hprev[c] : quad == 1 ? hprev[4 + c] : quad == 2 ? hprev[8 + c] : hprev[12 + c];
-      quadbuf = make_float4(hown[0], hown[1], hown[2], hown[3]);      // h_{t-1}[own quad] is next step's h_t
-      float da[4], dfp = 0.f;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float hn = fast_tanh(a[c]);
-        dfp += dh[c] * (hown[c] - hn);
-        da[c] = dh[c] * (1.f - ft) * (1.f - hn * hn);
-      }
-      dfp = warp_sum(dfp);
-      if (lane == 0) dfpart[t][warp] = dfp;
-      // full da row of this k
-      float darow[VD];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) darow[j * 4 + c] = __shfl_sync(0xffffffffu, da[c], (lane & ~3) + j);
-      // dk_t[k] = da[k,:] . v_t
-      if (quad == 0) {
-        float s = 0.f;
-#pragma unroll
-        for (int j = 0; j < VD; ++j) s += darow[j] * vs[t][j];
-        dks[t][lrow] = s;
-      }
-      // dv_t[v] = sum_k da[k,v] k_t[k]  (own columns; reduce over the 8 rows of this warp)
-      float dvp[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        dvp[c] = da[c] * kt;
-        dvp[c] += __shfl_xor_sync(0xffffffffu, dvp[c], 4);
-        dvp[c] += __shfl_xor_sync(0xffffffffu, dvp[c], 8);
-        dvp[c] += __shfl_xor_sync(0xffffffffu, dvp[c], 16);
-      }
-      if (lane < 4) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) dvpart[t][warp][quad * 4 + c] = dvp[c];
-      }
-      // dW[u,v] += h_{t-1}[k,u] da[k,v]  for own u = 4*quad + c
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const float hu = hown[c];
-#pragma unroll
-        for (int j = 0; j < VD; ++j) P[c][j] += hu * darow[j];
-      }
-      // dh_{t-1}[k,u] = f dh_t[k,u] + sum_v da[k,v] W[u,v]   for own u
-#pragma unroll
-      for (int c = 0; c < 4; ++c) dh[c] *= ft;
-#pragma unroll
-      for (int j = 0; j < VD; ++j) {
-        const float4 w = *reinterpret_cast<const float4*>(&Wt[j][quad * 4]);   // W[u=4q..4q+3][v=j]
-        dh[0] += darow[j] * w.x; dh[1] += darow[j] * w.y; dh[2] += darow[j] * w.z; dh[3] += darow[j] * w.w;
-      }
-    }
-    __syncthreads();
-    // write this block's per-step gradients
-    for (int e = tid; e < nt * RS; e += NT) {
-      const int t = e / RS, c = e % RS;
-      dq_h[((size_t)(b * S + t0 + t) * H + h) * KD + sp * RS + c] = dqs[t][c];
-      dk_h[((size_t)(b * S + t0 + t) * H + h) * KD + sp * RS + c] = dks[t][c];
+    for (int i = 0; i < 4; ++i) dw_sum[n][i] = 0.f;
+  in.fetch((nblocks - 1) * TB, tid);
+  in.commit(sh.stage[(nblocks - 1) & 1], tid);
+  const int col = reduced_col(lane);
+  auto write_out = [&](int blk) {                 // the gradients of block `blk` from its shared-memory parts
+    const int t0 = blk * TB, nt = min(TB, S - t0), p = blk & 1;
+    for (int e = tid; e < nt * KD; e += NT) {
+      const size_t o = ((size_t)(b * S + t0 + e / KD) * H + h) * KD + e % KD;
+      dq_h[o] = sh.dq[p][e / KD][e % KD];
+      dk_h[o] = sh.dk[p][e / KD][e % KD];
     }
     for (int e = tid; e < nt * VD; e += NT) {
-      const int t = e / VD, c = e % VD;
       float s = 0.f;
 #pragma unroll
-      for (int w = 0; w < NW; ++w) s += dvpart[t][w][c];
-      float* dst = dv + ((size_t)(b * S + t0 + t) * H + h) * VD + c;
-      if (SPLITS == 1) *dst = s; else atomicAdd(dst, s);
+      for (int i = 0; i < NW; ++i) s += sh.dv[p][e / VD][i][e % VD];
+      dv[((size_t)(b * S + t0 + e / VD) * H + h) * VD + e % VD] = s;
     }
-    if (tid < nt) {
+    for (int e = tid; e < TB * 8; e += NT) {      // eight threads per step
+      const int t = e >> 3, part = e & 7;
       float s = 0.f;
+      if (t < nt) {
 #pragma unroll
-      for (int w = 0; w < NW; ++w) s += dfpart[tid][w];
-      float* dst = df + (size_t)(b * S + t0 + tid) * H + h;
-      if (SPLITS == 1) *dst = s; else atomicAdd(dst, s);
-    }
-    __syncthreads();
-  }
-  // reduce dW over the rows k of this CTA, then over batch with atomics
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-#pragma unroll
-    for (int j = 0; j < VD; ++j) {
-      float s = P[c][j];
+        for (int i = 0; i < NT / 8; ++i) s += sh.df[p][t][part + 8 * i];
+      }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
       s += __shfl_xor_sync(0xffffffffu, s, 4);
-      s += __shfl_xor_sync(0xffffffffu, s, 8);
-      s += __shfl_xor_sync(0xffffffffu, s, 16);
-      if (lane < 4) atomicAdd(&dWs[quad * 4 + c][j], s);
+      if (part == 0 && t < nt) df[(size_t)(b * S + t0 + t) * H + h] = s;
     }
+  };
+  for (int blk = nblocks - 1; blk >= 0; --blk) {
+    __syncthreads();                              // inputs of this block and gradient parts of the previous one are complete
+    const int p = blk & 1;
+    const Stage<KD, true>& st = sh.stage[p];
+    if (blk > 0) in.fetch((blk - 1) * TB, tid);
+    if (blk + 1 < nblocks) write_out(blk + 1);
+    const int t0 = blk * TB;
+    float dw_blk[2][4];                           // this block's part of dW: added to the running sum once per block
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dw_blk[n][i] = 0.f;
+#pragma unroll 1
+    for (int t1 = TB - AHEAD; t1 >= 0; t1 -= AHEAD) {
+#pragma unroll
+      for (int sl = AHEAD - 1; sl >= 0; --sl) {
+        const int t = t1 + sl;
+        float hprev[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) hprev[i] = ring[sl][i];
+        load_state(ring[sl], t0 + t - 1 - AHEAD);
+        if (t0 + t >= S) continue;                // past the end: the whole CTA skips
+        const float k0 = st.k[t][r0], k1 = st.k[t][r0 + 8], q0 = st.q[t][r0], q1 = st.q[t][r0 + 8], ft = st.f[t];
+        const float2 va = *reinterpret_cast<const float2*>(&st.v[t][2 * t4]), vb = *reinterpret_cast<const float2*>(&st.v[t][8 + 2 * t4]);
+        const float2 ga = *reinterpret_cast<const float2*>(&st.g[t][2 * t4]), gb = *reinterpret_cast<const float2*>(&st.g[t][8 + 2 * t4]);
+        const float vv[4] = {va.x, va.y, vb.x, vb.y}, gg[4] = {ga.x, ga.y, gb.x, gb.y};
+        // replay of tanh(a_t); off the chain
+        Split3 sp;
+        split3(hprev, sp);
+        float a[8];
+        times16(a, sp, w);
+        float da[8], dfp = 0.f, red[4] = {0.f, 0.f, 0.f, 0.f};      // red: dq of rows r0, r0 + 8, dk of the same
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int c = (i >> 2) * 2 + (i & 1), up = (i >> 1) & 1;
+          const float hn = fast_tanh(fmaf(up ? k1 : k0, vv[c], a[i]));
+          dh[i] = fmaf(up ? q1 : q0, gg[c], dh[i]);
+          red[up] = fmaf(hcur[i], gg[c], red[up]);
+          dfp = fmaf(dh[i], hprev[i] - hn, dfp);
+          da[i] = dh[i] * ((1.f - ft) * (1.f - hn * hn));
+          red[2 + up] = fmaf(da[i], vv[c], red[2 + up]);
+        }
+        Split3 sd;
+        split3(da, sd);
+        float back[8];
+        times16(back, sd, wt);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dh[i] = fmaf(ft, dh[i], back[i]);
+        // dW[u][v] += sum_rows h_{t-1}[row][u] da[row][v]: both factors transposed within the warp, six products of parts
+        {
+          uint32_t ht[3][4], dt[3][4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int j = (i & 1) * 2 + (i >> 1);  // block (row half, column half) -> (column half, row half)
+            ht[0][j] = transpose8x8(sp.hi[i]); ht[1][j] = transpose8x8(sp.mid[i]); ht[2][j] = transpose8x8(sp.lo[i]);
+            dt[0][i] = transpose8x8(sd.hi[i]); dt[1][i] = transpose8x8(sd.mid[i]); dt[2][i] = transpose8x8(sd.lo[i]);
+          }
+#pragma unroll
+          for (int n = 0; n < 2; ++n) {
+#pragma unroll
+            for (int x = 2; x >= 0; --x)
+#pragma unroll
+              for (int z = 2 - x; z >= 0; --z) {
+                const uint32_t bb[2] = {dt[z][n * 2], dt[z][n * 2 + 1]};
+                mma16816(dw_blk[n], ht[x], bb);
+              }
+          }
+        }
+        // dq, dk: sum over the four lanes of a row; each lane ends with one of the four
+        {
+          const bool o1 = lane & 1, o2 = lane & 2;
+          const float x0 = (o1 ? red[2] : red[0]) + __shfl_xor_sync(0xffffffffu, o1 ? red[0] : red[2], 1);
+          const float x1 = (o1 ? red[3] : red[1]) + __shfl_xor_sync(0xffffffffu, o1 ? red[1] : red[3], 1);
+          const float r = (o2 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, o2 ? x0 : x1, 2);
+          (o1 ? sh.dk : sh.dq)[p][t][r0 + (o2 ? 8 : 0)] = r;
+        }
+        float dvp[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const int i = (c >> 1) * 4 + (c & 1);
+          dvp[c] = fmaf(da[i + 2], k1, da[i] * k0);
+        }
+        const float r = reduce_rows4(dvp, lane);
+        if ((lane & 4) == 0) sh.dv[p][t][warp][col] = r;
+        sh.df[p][t][tid] = dfp;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) hcur[i] = hprev[i];
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dw_sum[n][i] += dw_blk[n][i];
+    if (blk > 0) in.commit(sh.stage[(blk - 1) & 1], tid);
+  }
   __syncthreads();
-  for (int i = tid; i < VD * VD; i += NT) atomicAdd(dW + (size_t)h * VD * VD + i, dWs[i / VD][i % VD]);
+  write_out(0);
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) atomicAdd(&sh.dw[g + ((i & 2) ? 8 : 0)][n * 8 + 2 * t4 + (i & 1)], dw_sum[n][i]);
+  __syncthreads();
+  for (int i = tid; i < VD * VD; i += NT) atomicAdd(dW + (size_t)h * VD * VD + i, (&sh.dw[0][0])[i]);
+}
+
+template <int KD>
+static int launch_bwd(const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v, const __nv_bfloat16* W, const float* f,
+                      const float* hist, const __nv_bfloat16* dy, float* dq_h, float* dk_h, float* dv, float* df, float* dW, int B, int S,
+                      int H, int Hq, int Hk, bool vec, cudaStream_t s) {
+  static PerDevice cfg;
+  if (cfg.first()) {
+    if (cudaFuncSetAttribute(m2rnn_bwd_kernel<KD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdShared<KD>)) != cudaSuccess)
+      return -2;
+    cfg.done();
+  }
+  m2rnn_bwd_kernel<KD><<<B * H, KD * 2, sizeof(BwdShared<KD>), s>>>(q, k, v, W, f, hist, dy, dq_h, dk_h, dv, df, dW, S, H, Hq, Hk, vec);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
 }  // namespace cm
 
 using namespace cm;
 
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 // q [B,S,Hq,KD], k [B,S,Hk,KD], v [B,S,H,16], W [H,16,16] (bf16); f [B,S,H] fp32.
-// y [B,S,H,16] bf16; y_part: fp32 scratch [KD/16,B,S,H,16] (needed for KD > 16, may be null otherwise);
-// hist (nullable) [B,H,S,KD,16] fp32; h_last (nullable) [B,H,KD,16] fp32.
-extern "C" int cm_m2rnn_fwd(const void* q, const void* k, const void* v, const void* W, const float* f, void* y,
-                            float* y_part, float* hist, float* h_last, int B, int S, int H, int Hq, int Hk, int KD, int VDim,
-                            cudaStream_t s) {
+// y [B,S,H,16] bf16; hist (nullable) [B,H,S,KD,16] fp32; h_last (nullable) [B,H,KD,16] fp32.
+extern "C" int cm_m2rnn_fwd(const void* q, const void* k, const void* v, const void* W, const float* f, void* y, float* hist, float* h_last,
+                            int B, int S, int H, int Hq, int Hk, int KD, int VDim, cudaStream_t s) {
   if (B <= 0 || S <= 0) return 0;
   if (VDim != VD) return -10;
   auto qp = (const __nv_bfloat16*)q; auto kp = (const __nv_bfloat16*)k; auto vp = (const __nv_bfloat16*)v;
   auto wp = (const __nv_bfloat16*)W; auto yp = (__nv_bfloat16*)y;
-  const int bh = B * H;
-  if (KD == 64 || KD == 32) {
-    const int splits = KD / 16;
-    if (!y_part) return -10;          // several CTAs per head: needs the [KD/16, B, S, H, 16] fp32 partial buffer
-    if (KD == 64) m2rnn_fwd_kernel<64><<<bh * splits, 64, 0, s>>>(qp, kp, vp, wp, f, yp, y_part, hist, h_last, B, S, H, Hq, Hk);
-    else m2rnn_fwd_kernel<32><<<bh * splits, 64, 0, s>>>(qp, kp, vp, wp, f, yp, y_part, hist, h_last, B, S, H, Hq, Hk);
-    const long long n = (long long)B * S * H * VD;
-    long long blocks = (n + 255) / 256;
-    const int grid = (int)(blocks < (long long)sm_count() * 8 ? blocks : (long long)sm_count() * 8);
-    m2rnn_sum_parts_kernel<<<grid, 256, 0, s>>>(y_part, yp, splits, n);
-  } else if (KD == 16) {
-    m2rnn_fwd_kernel<16><<<bh, 64, 0, s>>>(qp, kp, vp, wp, f, yp, y_part, hist, h_last, B, S, H, Hq, Hk);
-  } else {
-    return -10;
-  }
+  const bool vec = aligned16(q) && aligned16(k) && aligned16(v);
+  if (KD == 64) m2rnn_fwd_kernel<64><<<B * H, 128, 0, s>>>(qp, kp, vp, wp, f, yp, hist, h_last, S, H, Hq, Hk, vec);
+  else if (KD == 32) m2rnn_fwd_kernel<32><<<B * H, 64, 0, s>>>(qp, kp, vp, wp, f, yp, hist, h_last, S, H, Hq, Hk, vec);
+  else if (KD == 16) m2rnn_fwd_kernel<16><<<B * H, 32, 0, s>>>(qp, kp, vp, wp, f, yp, hist, h_last, S, H, Hq, Hk, vec);
+  else return -10;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// dq_h, dk_h [B,S,H,KD] fp32 (per head); dv [B,S,H,16], df [B,S,H] and dW [H,16,16] fp32 are accumulated: the caller zeroes them.
+// dq_h, dk_h [B,S,H,KD] fp32 (per head), dv [B,S,H,16] and df [B,S,H] fp32 are written; dW [H,16,16] fp32 is accumulated over
+// the batch: the caller zeroes it.
 extern "C" int cm_m2rnn_bwd(const void* q, const void* k, const void* v, const void* W, const float* f, const float* hist,
                             const void* dy, float* dq_h, float* dk_h, float* dv, float* df, float* dW, int B, int S, int H,
                             int Hq, int Hk, int KD, int VDim, cudaStream_t s) {
@@ -420,12 +472,9 @@ extern "C" int cm_m2rnn_bwd(const void* q, const void* k, const void* v, const v
   if (VDim != VD) return -10;
   auto qp = (const __nv_bfloat16*)q; auto kp = (const __nv_bfloat16*)k; auto vp = (const __nv_bfloat16*)v;
   auto wp = (const __nv_bfloat16*)W; auto gp = (const __nv_bfloat16*)dy;
-  const int grid = B * H;
-  // K = 64: four CTAs of 16 state rows each per (batch, head) (6.3 ms against 6.6 ms with two CTAs of 32 rows and 10.4 ms
-  // with one CTA of 64 rows at B 4, S 4096, 51 heads): more resident CTAs hide the per-step dependency chain better
-  if (KD == 64) m2rnn_bwd_kernel<64, 16><<<grid * 4, 64, 0, s>>>(qp, kp, vp, wp, f, hist, gp, dq_h, dk_h, dv, df, dW, S, H, Hq, Hk);
-  else if (KD == 32) m2rnn_bwd_kernel<32, 32><<<grid, 128, 0, s>>>(qp, kp, vp, wp, f, hist, gp, dq_h, dk_h, dv, df, dW, S, H, Hq, Hk);
-  else if (KD == 16) m2rnn_bwd_kernel<16, 16><<<grid, 64, 0, s>>>(qp, kp, vp, wp, f, hist, gp, dq_h, dk_h, dv, df, dW, S, H, Hq, Hk);
-  else return -10;
-  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  const bool vec = aligned16(q) && aligned16(k) && aligned16(v) && aligned16(dy);
+  if (KD == 64) return launch_bwd<64>(qp, kp, vp, wp, f, hist, gp, dq_h, dk_h, dv, df, dW, B, S, H, Hq, Hk, vec, s);
+  if (KD == 32) return launch_bwd<32>(qp, kp, vp, wp, f, hist, gp, dq_h, dk_h, dv, df, dW, B, S, H, Hq, Hk, vec, s);
+  if (KD == 16) return launch_bwd<16>(qp, kp, vp, wp, f, hist, gp, dq_h, dk_h, dv, df, dW, B, S, H, Hq, Hk, vec, s);
+  return -10;
 }

@@ -191,3 +191,35 @@ def test_ssd_variant_mixers_on_gpu_match_the_cpu_fp32_module(variant):
         assert F_.launch_counts().get("causal_conv1d_silu", 0) == 1
     assert _rel(yg.cpu(), yr) < 4e-2
     assert _rel(xg.grad.cpu(), xr.grad) < 6e-2
+
+
+@pytest.mark.parametrize("B,S,H,KD,shared,offset", [(1, 1, 2, 64, True, 0), (2, 16, 3, 64, False, 0), (1, 33, 5, 32, True, 0),
+                                                    (2, 50, 2, 64, True, 1), (1, 19, 3, 16, False, 3)])
+def test_m2rnn_blocks_and_unaligned_inputs(B, S, H, KD, shared, offset):
+    """Sequence lengths at, below and past the 16-step staging block, and inputs whose storage starts off a 16-byte boundary.
+    The state factor is fp32 (three bf16 parts per factor): the fp32 gradient of f agrees to the accuracy of tanh.approx
+    (2^-11 of tanh, less in the mean)."""
+    from cppmega_b200.ops import reference as ref
+    from cppmega_b200.ops.cuda import kernels2
+    torch.manual_seed(S)
+    Hq = 1 if shared else H
+
+    def make(*shape, std):
+        buf = (torch.randn(offset + torch.Size(shape).numel(), device="cuda") * std).bfloat16()
+        return buf[offset:].view(shape).detach().requires_grad_()
+
+    q, k, v = make(B, S, Hq, KD, std=0.5), make(B, S, Hq, KD, std=0.5), make(B, S, H, 16, std=0.5)
+    W = make(H, 16, 16, std=0.3)
+    f = torch.rand(B, S, H, device="cuda").requires_grad_()
+    y = kernels2.m2rnn_scan(q, k, v, W, f)
+    g = torch.randn_like(y)
+    y.backward(g)
+    refs = [t.detach().float().requires_grad_() for t in (q, k, v, W, f)]
+    yr, _ = ref.m2rnn_scan(*refs)
+    yr.backward(g.float())
+    assert _rel(y, yr) < 5e-3
+    for name, a, b in zip("q k v W f".split(), (q, k, v, W, f), refs):
+        if b.grad.norm() > 0:
+            assert _rel(a.grad, b.grad) < (1e-3 if name == "f" else 5e-3), name
+        else:
+            assert a.grad.norm() == 0, name
