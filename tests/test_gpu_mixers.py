@@ -223,3 +223,29 @@ def test_m2rnn_blocks_and_unaligned_inputs(B, S, H, KD, shared, offset):
             assert _rel(a.grad, b.grad) < (1e-3 if name == "f" else 5e-3), name
         else:
             assert a.grad.norm() == 0, name
+
+
+@pytest.mark.parametrize("B,S,H,std,scale", [(1, 128, 1, 0.7, 0.09), (1, 384, 2, 4.0, 0.09), (2, 640, 1, 0.7, -0.05), (1, 256, 3, 0.7, 0.0)])
+def test_dense_causal_attention_tile_pairs(B, S, H, std, scale):
+    """Odd and even counts of query tiles (the last pair has one or two), scores large enough that the running maximum grows
+    past the rescale threshold between key tiles, and scales without a sign."""
+    from cppmega_b200.ops import cuda as cu
+    from cppmega_b200.ops import functional as F_
+    torch.manual_seed(S)
+    grow = torch.linspace(0.2, 1.0, S, device="cuda").view(1, S, 1, 1)          # later keys score higher
+    q = (torch.randn(B, S, H, 128, device="cuda") * std).bfloat16().requires_grad_()
+    k = (torch.randn(B, S, H, 128, device="cuda") * std * grow).bfloat16().requires_grad_()
+    v = torch.randn(B, S, H, 64, device="cuda").bfloat16().requires_grad_()
+    o = F_.causal_attention(q, k, v, scale)
+    g = torch.randn_like(o)
+    o.backward(g)
+    cu.check_errors()
+    qr, kr, vr = (t.detach().float().requires_grad_() for t in (q, k, v))
+    orf = _attn_ref(qr, kr, vr, scale)
+    orf.backward(g.float())
+    assert _rel(o, orf) < 1e-2
+    for name, a, b in (("dq", q.grad, qr.grad), ("dk", k.grad, kr.grad), ("dv", v.grad, vr.grad)):
+        if b.norm() > 0:
+            assert _rel(a, b) < 1.5e-2, name
+        else:
+            assert a.norm() == 0, name
