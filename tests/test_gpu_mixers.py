@@ -249,3 +249,34 @@ def test_dense_causal_attention_tile_pairs(B, S, H, std, scale):
             assert _rel(a, b) < 1.5e-2, name
         else:
             assert a.norm() == 0, name
+
+
+@pytest.mark.parametrize("B,S", [(1, 40), (2, 300)])
+def test_sparse_mla_repeated_and_masked_keys(B, S):
+    """Rows selected twice by one query, queries with few or no keys, and keys after the query: the gradient rows of a key are
+    summed over all of its uses."""
+    from cppmega_b200.ops import cuda as cu
+    from cppmega_b200.ops import reference as ref
+    from cppmega_b200.ops.cuda import kernels4
+    torch.manual_seed(S)
+    q = (torch.randn(B, S, 32, 128, device="cuda") * 0.5).bfloat16().requires_grad_()
+    kv = (torch.randn(B, S, 128, device="cuda") * 0.5).bfloat16().requires_grad_()
+    idx = torch.randint(-60, S, (B, S, 256), device="cuda").clamp_min(-1).to(torch.int32)
+    idx[:, 3] = -1
+    idx[:, 5, 1:] = -1
+    o = kernels4.sparse_mla(q, kv, idx, 0.1, 64)
+    g = torch.randn_like(o)
+    o.backward(g)
+    cu.check_errors()
+    # the definition has no gradient for a query without keys: give it one key there and no upstream gradient
+    some, gr = idx.clone(), g.float().clone()
+    some[:, 3, 0] = 0
+    gr[:, 3] = 0
+    qr, kr = (t.detach().float().requires_grad_() for t in (q, kv))
+    orf, _ = ref.sparse_mla(qr, kr, some, 0.1, 64)
+    orf.backward(gr)
+    assert o[:, 3].norm() == 0
+    live = torch.arange(S, device="cuda") != 3
+    assert _rel(o[:, live], orf[:, live]) < 1e-2
+    assert _rel(q.grad, qr.grad) < 1.5e-2
+    assert _rel(kv.grad, kr.grad) < 1.5e-2
