@@ -15,6 +15,7 @@ def declare(L: ctypes.CDLL) -> None:
     vp, i32, i64 = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong
     sig = {
         "cm_ce_fwd_bwd": [vp, vp, vp, vp, vp, i32, i32, i64, i32, i32, vp],
+        "cm_scale_to_bf16": [vp, i32, vp, vp, i64, vp],
     }
     for name, args in sig.items():
         fn = getattr(L, name, None)
@@ -131,7 +132,8 @@ class LinearCEWeightedFn(torch.autograd.Function):
         need_grad = h.requires_grad or w.requires_grad
         per_tok = torch.empty(T, dtype=torch.float32, device=h.device)
         dh = torch.empty_like(h) if need_grad else None
-        dw = torch.zeros(V, H, dtype=torch.float32, device=h.device) if need_grad else None
+        # the first chunk's product writes dw, the others add to it
+        dw = (torch.empty if T > 0 else torch.zeros)(V, H, dtype=torch.float32, device=h.device) if need_grad else None
         labels = labels.to(torch.int64).contiguous()
         weights = weights.to(torch.float32).contiguous()
         C = LinearCEWeightedFn.CHUNK
@@ -147,7 +149,7 @@ class LinearCEWeightedFn(torch.autograd.Function):
             F_.count_launch("cross_entropy")
             if need_grad:
                 gemm(lg, w, b_mn=True, out=dh[s:e])
-                gemm(lg, h[s:e], a_mn=True, b_mn=True, out=dw, accumulate=True)
+                gemm(lg, h[s:e], a_mn=True, b_mn=True, out=dw, accumulate=s > 0)
         total = (per_tok * weights).sum()
         if need_grad:
             ctx.save_for_backward(dh, dw)
@@ -157,8 +159,19 @@ class LinearCEWeightedFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g_total, _g_per_tok):
+        from . import lib, stream_ptr, _check
         dh, dw = ctx.saved_tensors
-        return dh * g_total.to(dh.dtype), (dw * g_total).to(ctx.w_dtype), None, None, None
+        if torch.is_grad_enabled():                    # create_graph: keep the product with the upstream factor differentiable
+            return dh * g_total.to(dh.dtype), (dw * g_total).to(ctx.w_dtype), None, None, None
+        g = g_total.float().reshape(1)
+        outs = []
+        for t in (dh, dw):                             # scaled and rounded to bf16 in one pass
+            o = torch.empty(t.shape, dtype=torch.bfloat16, device=t.device)
+            _check(lib().cm_scale_to_bf16(t.data_ptr(), int(t.dtype == torch.float32), o.data_ptr(), g.data_ptr(), t.numel(),
+                                          stream_ptr()), "cm_scale_to_bf16")
+            F_.count_launch("scale_to_bf16")
+            outs.append(o)
+        return outs[0], outs[1], None, None, None
 
 
 def linear_cross_entropy_weighted(h, w, labels, weights, ignore_index):

@@ -26,6 +26,19 @@ def test_rmsnorm(rows, H):
     assert _rel(w.grad, wr.grad) < 8e-3
 
 
+@pytest.mark.parametrize("n", [8, 8 * 1023, 8 * 512 * 148 * 8 + 8])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_scale_to_bf16(n, dtype):
+    """The same bits as the product and cast of the tensor library."""
+    from cppmega_b200.ops import cuda as cu
+    torch.manual_seed(n)
+    x = torch.randn(n, device="cuda").to(dtype)
+    g = torch.tensor([0.37], device="cuda")
+    out = torch.empty(n, dtype=torch.bfloat16, device="cuda")
+    assert cu.lib().cm_scale_to_bf16(x.data_ptr(), int(dtype == torch.float32), out.data_ptr(), g.data_ptr(), n, cu.stream_ptr()) == 0
+    assert torch.equal(out, (x * g.to(dtype)).to(torch.bfloat16))
+
+
 def test_swiglu():
     from cppmega_b200.ops import cuda as cu, reference as ref
     torch.manual_seed(0)
@@ -83,3 +96,10 @@ def test_linear_ce_weighted(T, H, V):
     assert abs(total.item() - tr.item()) < 2e-2 * abs(tr.item()) + 1e-3
     assert _rel(h.grad, hr.grad) < 3e-2
     assert _rel(w.grad, wr.grad) < 3e-2
+
+
+@pytest.mark.parametrize("T,H,V", [(33, 64, 8), (130, 64, 16392), (4097, 64, 512)])
+def test_linear_ce_chunk_and_vocabulary_edges(T, H, V):
+    """A vocabulary of one vector, one that ends inside an unrolled group of vectors, and a last chunk of one row (the first
+    chunk writes dw, the second adds to it)."""
+    test_linear_ce_weighted(T, H, V)
