@@ -19,12 +19,18 @@
 namespace cm {
 namespace mx {
 
+// ceil(log2(amax / 448)) + 127 from the bits of the quotient: its exponent field, one more unless it is a power of two (a bf16
+// amax makes it one only for 224 * 2^k, whose product with fl(1/448) rounds to the power of two itself).
 __device__ __forceinline__ uint8_t e8m0_from_amax(float amax) {
   if (!(amax > 0.f)) return 127;
-  int e = (int)ceilf(log2f(amax * (1.f / 448.f))) + 127;
+  const uint32_t u = __float_as_uint(amax * (1.f / 448.f));
+  int e = (int)(u >> 23) + ((u & 0x7fffffu) != 0);
+  if (e == 255) return 1;                         // an infinity has no scale
   e = e < 1 ? 1 : (e > 254 ? 254 : e);
   return (uint8_t)e;
 }
+// 2^(127 - sb), sb in 1..254
+__device__ __forceinline__ float inverse_scale(uint8_t sb) { return __uint_as_float(sb == 254 ? 0x00400000u : (254u - sb) << 23); }
 // two floats -> two e4m3 bytes (lo in bits 0..7)
 __device__ __forceinline__ uint16_t to_e4m3x2(float lo, float hi) {
   uint16_t r;
@@ -67,7 +73,7 @@ __global__ void __launch_bounds__(256) quantize_rowwise_kernel(const __nv_bfloat
     am = fmaxf(am, __shfl_xor_sync(live, am, 1));
     am = fmaxf(am, __shfl_xor_sync(live, am, 2));
     const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
-    const float mult = exp2f(127.f - (float)sb);
+    const float mult = inverse_scale(sb);
     uint2 o;
     o.x = (uint32_t)to_e4m3x2(f[0] * mult, f[1] * mult) | ((uint32_t)to_e4m3x2(f[2] * mult, f[3] * mult) << 16);
     o.y = (uint32_t)to_e4m3x2(f[4] * mult, f[5] * mult) | ((uint32_t)to_e4m3x2(f[6] * mult, f[7] * mult) << 16);
@@ -97,7 +103,7 @@ __global__ void __launch_bounds__(128) quantize_colwise_kernel(const __nv_bfloat
     am = fmaxf(am, fabsf(f[r]));
   }
   const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
-  const float mult = exp2f(127.f - (float)sb);
+  const float mult = inverse_scale(sb);
   uint32_t w[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q)
@@ -109,81 +115,121 @@ __global__ void __launch_bounds__(128) quantize_colwise_kernel(const __nv_bfloat
   if (sw) sw[swizzled_index(c, (int)blockIdx.y, (int)((rows / 32 + 3) / 4))] = sb;
 }
 
-// Both orientations from one read of x: CTA = tile of 32 rows x 256 columns.  Phase 1 is the row-wise kernel (8 values
-// per thread, 4 threads per block) and parks the values as fp32 in shared memory; phase 2 walks the columns of the tile.
-// The tile is stored column-permuted (logical column 8 v + j at physical column 32 j + v) with a row stride of 257 floats,
-// which makes both the phase-1 stores and the phase-2 column reads bank-conflict free.
+// Both orientations from one read of x: CTA = tile of 128 rows x 128 columns.  Phase 1 is the row-wise kernel (8 values per
+// thread, 4 threads per block) and parks the raw values in shared memory; in phase 2 a thread takes two neighbouring columns
+// of one 32-row block, so a bank word is one read.  A tile is one line (128 bytes) of every row and of every transposed row,
+// and exactly one 128x4 scale tile of each orientation, which leaves as whole words.  Memory-bound; with 32 x 256 tiles of
+// fp32 in shared memory, 32-byte transposed runs and log2 / exp2 per block, 8192 x 8192
+// and 8192 x 4096 together took 201 us; now 169.
+constexpr int QB_LD = 65;                                   // words per row of 128 bf16; each 32-row block is 8 words further
+__device__ __forceinline__ int qb_word(int row, int pair) { return row * QB_LD + (row >> 5) * 8 + pair; }
+
 __global__ void __launch_bounds__(256) quantize_both_kernel(const __nv_bfloat16* __restrict__ x, uint8_t* __restrict__ pay_r,
                                                             uint8_t* __restrict__ sc_r, uint8_t* __restrict__ sw_r,
                                                             uint8_t* __restrict__ pay_t, uint8_t* __restrict__ sc_t,
                                                             uint8_t* __restrict__ sw_t, long long rows, int cols,
                                                             const float* __restrict__ tamax) {
-  __shared__ float tile[32][257];
-  const long long r0 = (long long)blockIdx.y * 32;
-  const int c0 = blockIdx.x * 256;
+  __shared__ uint32_t tile[128 * QB_LD + 32];
+  __shared__ __align__(4) uint8_t s_r[128][4], s_t[128][4];
+  const long long r0 = (long long)blockIdx.y * 128;
+  const int c0 = blockIdx.x * 128;
+  const int nrows = (int)min(128ll, rows - r0), ncols = min(128, cols - c0);        // multiples of 32
   const int kb_row = cols / 32, kbt_row = (kb_row + 3) / 4;
   const int kb_col = (int)(rows / 32), kbt_col = (kb_col + 3) / 4;
-  const int lane = threadIdx.x & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  uint4 raw[8];
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int row = it * 8 + (threadIdx.x >> 5);
-    const int col = c0 + lane * 8;
-    const bool valid = col < cols;
-    float f[8];
-    float am = 0.f;
-    if (valid) {
-      const uint4 raw = *reinterpret_cast<const uint4*>(x + (size_t)(r0 + row) * cols + col);
-      const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  for (int it = 0; it < 8; ++it) {
+    const int row = it * 16 + (tid >> 4), v = tid & 15;
+    raw[it] = make_uint4(0, 0, 0, 0);
+    if (row < nrows && v * 8 < ncols) raw[it] = *reinterpret_cast<const uint4*>(x + (size_t)(r0 + row) * cols + c0 + v * 8);
+  }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 t = __bfloat1622float2(b[j]);
-        f[2 * j] = t.x; f[2 * j + 1] = t.y;
-        am = fmaxf(am, fmaxf(fabsf(t.x), fabsf(t.y)));
-      }
-    } else {
+  for (int it = 0; it < 8; ++it) {
+    const int row = it * 16 + (tid >> 4), v = tid & 15;
+    const __nv_bfloat162* b = reinterpret_cast<const __nv_bfloat162*>(&raw[it]);
+    float f[8], am = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = 0.f;
+    for (int j = 0; j < 4; ++j) {
+      const float2 t = __bfloat1622float2(b[j]);
+      f[2 * j] = t.x; f[2 * j + 1] = t.y;
+      am = fmaxf(am, fmaxf(fabsf(t.x), fabsf(t.y)));
     }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) tile[row][j * 32 + lane] = f[j];
+    uint32_t* w = &tile[qb_word(row, v * 4)];
+    w[0] = raw[it].x; w[1] = raw[it].y; w[2] = raw[it].z; w[3] = raw[it].w;
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-    if (valid) {
-      const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
-      const float mult = exp2f(127.f - (float)sb);
+    const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
+    const float mult = inverse_scale(sb);
+    if ((lane & 3) == 0) s_r[row][v >> 2] = sb;
+    if (row < nrows && v * 8 < ncols) {
       uint2 o;
       o.x = (uint32_t)to_e4m3x2(f[0] * mult, f[1] * mult) | ((uint32_t)to_e4m3x2(f[2] * mult, f[3] * mult) << 16);
       o.y = (uint32_t)to_e4m3x2(f[4] * mult, f[5] * mult) | ((uint32_t)to_e4m3x2(f[6] * mult, f[7] * mult) << 16);
-      *reinterpret_cast<uint2*>(pay_r + (size_t)(r0 + row) * cols + col) = o;
-      if ((lane & 3) == 0) {
-        const int kb = col >> 5;
-        sc_r[(size_t)(r0 + row) * kb_row + kb] = sb;
-        if (sw_r) sw_r[swizzled_index(r0 + row, kb, kbt_row)] = sb;
+      *reinterpret_cast<uint2*>(pay_r + (size_t)(r0 + row) * cols + c0 + v * 8) = o;
+    }
+  }
+  __syncthreads();
+  {
+    const int blk = lane & 3, pair = (tid >> 5) * 8 + (lane >> 2);        // 32-row block, column pair
+    uint32_t w[32];
+    float am[2] = {0.f, 0.f};
+#pragma unroll
+    for (int r = 0; r < 32; ++r) {
+      w[r] = tile[qb_word(blk * 32 + r, pair)];
+      am[0] = fmaxf(am[0], fabsf(__uint_as_float(w[r] << 16)));
+      am[1] = fmaxf(am[1], fabsf(__uint_as_float(w[r] & 0xffff0000u)));
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am[h]);
+      const float mult = inverse_scale(sb);
+      s_t[pair * 2 + h][blk] = sb;
+      uint32_t o[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        float f[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) f[j] = __uint_as_float(h ? (w[q * 4 + j] & 0xffff0000u) : (w[q * 4 + j] << 16)) * mult;
+        o[q] = (uint32_t)to_e4m3x2(f[0], f[1]) | ((uint32_t)to_e4m3x2(f[2], f[3]) << 16);
+      }
+      // neighbouring lanes hold neighbouring 32-byte blocks of the transposed row: they swap halves so that each of the two
+      // stores covers whole sectors
+      const bool odd = lane & 1;
+      uint4 got, a = make_uint4(o[0], o[1], o[2], o[3]), b = make_uint4(o[4], o[5], o[6], o[7]);
+      const uint4 give = odd ? a : b;
+      got.x = __shfl_xor_sync(0xffffffffu, give.x, 1); got.y = __shfl_xor_sync(0xffffffffu, give.y, 1);
+      got.z = __shfl_xor_sync(0xffffffffu, give.z, 1); got.w = __shfl_xor_sync(0xffffffffu, give.w, 1);
+      const int col = pair * 2 + h, even_blk = blk & 2;
+      if (col < ncols) {
+        uint8_t* dst = pay_t + (size_t)(c0 + col) * rows + r0 + even_blk * 32 + (odd ? 16 : 0);
+        if (even_blk * 32 < nrows) *reinterpret_cast<uint4*>(dst) = odd ? got : a;                 // the even block
+        if (even_blk * 32 + 32 < nrows) *reinterpret_cast<uint4*>(dst + 32) = odd ? b : got;       // the odd block
       }
     }
   }
   __syncthreads();
-  const int p = threadIdx.x;                                // physical column of the tile
-  const int col = c0 + (p & 31) * 8 + (p >> 5);             // its logical column
-  if (col >= cols) return;
-  float f[32];
-  float am = 0.f;
-#pragma unroll
-  for (int r = 0; r < 32; ++r) {
-    f[r] = tile[r][p];
-    am = fmaxf(am, fabsf(f[r]));
+  // scales: thread < 128 one row, the others one column; whole words where all four blocks exist
+  const bool is_row = tid < 128;
+  const int k = tid & 127;
+  if (k < (is_row ? nrows : ncols)) {
+    const uint8_t* src = is_row ? s_r[k] : s_t[k];
+    const int nkb = (is_row ? ncols : nrows) / 32, kb0 = (is_row ? c0 : (int)r0) / 32, kbs = is_row ? kb_row : kb_col;
+    uint8_t* plain = (is_row ? sc_r + (size_t)(r0 + k) * kbs : sc_t + (size_t)(c0 + k) * kbs) + kb0;
+    uint8_t* sw = is_row ? sw_r : sw_t;
+    if (sw) sw += swizzled_index((is_row ? r0 : c0) + k, kb0, is_row ? kbt_row : kbt_col);
+    if (nkb == 4) {
+      const uint32_t v = *reinterpret_cast<const uint32_t*>(src);
+      if ((kbs & 3) == 0) *reinterpret_cast<uint32_t*>(plain) = v;
+      else for (int q = 0; q < 4; ++q) plain[q] = src[q];
+      if (sw) *reinterpret_cast<uint32_t*>(sw) = v;
+    } else {
+      for (int q = 0; q < nkb; ++q) {
+        plain[q] = src[q];
+        if (sw) sw[q] = src[q];
+      }
+    }
   }
-  const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
-  const float mult = exp2f(127.f - (float)sb);
-  uint32_t w[8];
-#pragma unroll
-  for (int q = 0; q < 8; ++q)
-    w[q] = (uint32_t)to_e4m3x2(f[4 * q] * mult, f[4 * q + 1] * mult) | ((uint32_t)to_e4m3x2(f[4 * q + 2] * mult, f[4 * q + 3] * mult) << 16);
-  uint4* dst = reinterpret_cast<uint4*>(pay_t + (size_t)col * rows + r0);
-  dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-  sc_t[(size_t)col * kb_col + blockIdx.y] = sb;
-  if (sw_t) sw_t[swizzled_index(col, (int)blockIdx.y, kbt_col)] = sb;
 }
 
 // absolute maximum of a bf16 tensor: non-negative floats order like their bit patterns, so an integer atomicMax works
@@ -279,7 +325,7 @@ extern "C" int cm_mxfp8_quantize_both(const void* x, void* pay_r, void* sc_r, vo
                                       long long rows, int cols, const float* tensor_amax, cudaStream_t s) {
   if (rows <= 0) return 0;
   if ((rows % 32) || (cols % 32)) return -10;
-  dim3 grid((cols + 255) / 256, (unsigned)(rows / 32));
+  dim3 grid((cols + 127) / 128, (unsigned)((rows + 127) / 128));
   quantize_both_kernel<<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, (uint8_t*)pay_r, (uint8_t*)sc_r, (uint8_t*)sw_r, (uint8_t*)pay_t,
                                            (uint8_t*)sc_t, (uint8_t*)sw_t, rows, cols, tensor_amax);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

@@ -500,3 +500,27 @@ def test_embedding_kernels_gather_and_scatter_add(grad_dtype):
         got = w.main_grad.float()
     tol = 2e-2 if grad_dtype != torch.float32 else 1e-3
     assert (got - wr.grad).norm() / wr.grad.norm() < tol
+
+
+@pytest.mark.parametrize("rows,cols", [(32, 32), (128, 128), (96, 416), (288, 160), (32, 1056)])
+def test_mxfp8_quantize_both_tile_edges(rows, cols):
+    """Payload and scale bytes of both orientations equal those of the one-orientation kernels and of the definition, at sizes
+    that end inside the 128 x 128 tile, with zero blocks and amax values at the powers of two of the scale rule."""
+    from cppmega_b200.ops import reference as ref
+    from cppmega_b200.ops.cuda import mxfp8
+    torch.manual_seed(rows + cols)
+    x = (torch.randn(rows, cols, device="cuda") * torch.exp2(torch.randint(-30, 30, (rows, 1), device="cuda").float())).bfloat16()
+    x[0, :32] = 0
+    x[1, :32] = 224.0
+    x[2, :32] = 448.0
+    x[3, :32] = 450.0
+    x[4, :32] = 2.0 ** -130
+    r, t = mxfp8.quantize_both(x)
+    for got, axis in ((r, 1), (t, 0)):
+        one = mxfp8.quantize_rowwise(x) if axis == 1 else mxfp8.quantize_colwise(x)
+        assert torch.equal(got.payload, one.payload) and torch.equal(got.scales, one.scales)
+        assert torch.equal(got.swizzled(), one.swizzled())
+        pay, sc = ref.mxfp8_quantize(x, axis)
+        pay, sc = (pay, sc) if axis == 1 else (pay.t(), sc.t())
+        assert torch.equal(got.scales, sc.contiguous())
+        assert torch.equal(got.payload, pay.contiguous().view(torch.uint8))
