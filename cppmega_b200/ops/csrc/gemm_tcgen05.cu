@@ -21,7 +21,11 @@
 // This replaces the reference's CUTLASS dense GEMM extension and its scalar grouped kernels
 // (cppmega/megatron/cuda_ext/cutlass_mxfp8_gemm.cu:56-360, cuda_ext/grouped_mxfp8_gemm.cu:61-234),
 // which have no sm_100 path.
+//
+// Problems with enough 256-row tiles go to the CTA-pair kernel of gemm_pair.cu (plan_dense below); this one keeps the small
+// dense problems (128- and 64-column tiles), experts with few rows, and the peer-memory modes.
 #include "common.cuh"
+#include "gemm_pair.cuh"
 
 namespace cm {
 
@@ -469,6 +473,58 @@ static int dispatch_layout(bool a_mn, bool b_mn, const CUtensorMap& tmA, const C
 
 using namespace cm;
 
+// Tile shape of a dense problem.  A launch takes ceil(tiles / tiles in flight) waves; the weight of a wave is its measured time
+// (16384 x 24960 x 4096: 24.2 us with 256 columns, 20.5 with 192, 17.8 with 128; one CTA 17.9 with 128 and 14.8 with 64):
+// narrow tiles read more operand bytes per product, so they only win where they save waves.
+struct DensePlan {
+  int pair, bn;
+};
+static DensePlan plan_dense(int M, int N, bool b_mn) {
+  const int sms = sm_count();
+  DensePlan best{1, 256};
+  double best_cost = 1e30;
+  auto consider = [&](int pair, int bn, double wave) {
+    const long long tiles = (long long)((M + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((N + bn - 1) / bn);
+    const long long slots = pair ? sms / 2 : sms;
+    const double cost = double((tiles + slots - 1) / slots) * wave;
+    if (cost < best_cost) { best_cost = cost; best = DensePlan{pair, bn}; }
+  };
+  consider(1, 256, 24.2);
+  if (!b_mn) consider(1, 192, 20.5);            // an MN-major B comes in runs of 64 columns per CTA
+  consider(1, 128, 17.8);
+  consider(0, 128, 17.9);
+  consider(0, 64, 14.8);
+  return best;
+}
+
+// cm_gemm_bf16 with the tile shape given: pair = 1: bn 128 or 256, with a K-major B also 192; pair = 0: bn 64 or 128.
+extern "C" int cm_gemm_bf16_tiled(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                                  long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate, int pair, int bn, int* err,
+                                  cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
+    return -10;   // TMA needs 16-byte aligned bases and row pitches
+  if (pair) {
+    if (!(bn == 256 || bn == 128 || (bn == 192 && !b_mn))) return -10;
+    const PairArgs args{M, N, K, bn, ldc, 1, accumulate, 0, nullptr, nullptr, err};
+    return launch_gemm_pair(PAIR_DENSE, a_mn, b_mn, out_fp32, A, B, C, lda, ldb, K, args, stream);
+  }
+  if (bn != 64 && bn != 128) return -10;
+  CUtensorMap tmA, tmB;
+  int rc = a_mn ? make_tmap_2d_bf16(&tmA, A, K, M, lda, 64) : make_tmap_2d_bf16(&tmA, A, M, K, lda, BM);
+  if (rc) return rc;
+  rc = b_mn ? make_tmap_2d_bf16(&tmB, B, K, N, ldb, 64) : make_tmap_2d_bf16(&tmB, B, N, K, ldb, bn);
+  if (rc) return rc;
+  GemmArgs args{M, N, K, ldc, 1, nullptr, nullptr, err, 0, 0, 0, 0, {}};
+  const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
+#define CM_DENSE(OUT, ACC_)                                                                                          \
+  (bn == 64 ? dispatch_layout<64, OUT, ACC_, DENSE>(a_mn, b_mn, tmA, tmB, (OUT*)C, args, tiles, stream)               \
+            : dispatch_layout<128, OUT, ACC_, DENSE>(a_mn, b_mn, tmA, tmB, (OUT*)C, args, tiles, stream))
+  if (out_fp32) return accumulate ? CM_DENSE(float, true) : CM_DENSE(float, false);
+  return accumulate ? CM_DENSE(__nv_bfloat16, true) : CM_DENSE(__nv_bfloat16, false);
+#undef CM_DENSE
+}
+
 // C[M,N] (+)= op(A) op(B).  a_mn: A is stored [K,M] (M contiguous) instead of [M,K]; b_mn: B is
 // stored [K,N] (N contiguous) instead of [N,K].  lda/ldb/ldc are row pitches in elements.
 // out_fp32: C is float (else bf16); accumulate: C += result.  `err` is a device int (may be null).
@@ -478,22 +534,18 @@ extern "C" int cm_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
     return -10;   // TMA needs 16-byte aligned bases and row pitches
-  CUtensorMap tmA, tmB;
-  int rc;
-  rc = a_mn ? make_tmap_2d_bf16(&tmA, A, K, M, lda, 64) : make_tmap_2d_bf16(&tmA, A, M, K, lda, BM);
-  if (rc) return rc;
-  constexpr int BN = 256;
-  rc = b_mn ? make_tmap_2d_bf16(&tmB, B, K, N, ldb, 64) : make_tmap_2d_bf16(&tmB, B, N, K, ldb, BN);
-  if (rc) return rc;
-  GemmArgs args{M, N, K, ldc, 1, nullptr, nullptr, err, 0, 0, 0, 0, {}};
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  if (out_fp32) {
-    if (accumulate) return dispatch_layout<BN, float, true, DENSE>(a_mn, b_mn, tmA, tmB, (float*)C, args, tiles, stream);
-    return dispatch_layout<BN, float, false, DENSE>(a_mn, b_mn, tmA, tmB, (float*)C, args, tiles, stream);
-  }
-  if (accumulate)
-    return dispatch_layout<BN, __nv_bfloat16, true, DENSE>(a_mn, b_mn, tmA, tmB, (__nv_bfloat16*)C, args, tiles, stream);
-  return dispatch_layout<BN, __nv_bfloat16, false, DENSE>(a_mn, b_mn, tmA, tmB, (__nv_bfloat16*)C, args, tiles, stream);
+  const DensePlan p = plan_dense(M, N, b_mn != 0);
+  return cm_gemm_bf16_tiled(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, p.pair, p.bn, err, stream);
+}
+
+// Expert segments start at multiples of 128 rows, so a 256-row pair tile at a segment boundary is worked on twice.  From a
+// mean of four 128-row tiles per expert on that costs less than the pair gains; below it the one-CTA kernel stays.
+static bool pair_for_experts(int rows, int num_experts) { return rows >= num_experts * 5 * BM; }
+// Fewest column tiles, weighted by their time as in plan_dense.
+static int expert_bn(int N, bool b_mn) {
+  const int n256 = (N + 255) / 256, n192 = (N + 191) / 192, n128 = (N + 127) / 128;
+  if (!b_mn && n192 * 20.5 < n256 * 24.2 && n192 * 20.5 <= n128 * 17.8) return 192;
+  return n128 * 17.8 < n256 * 24.2 ? 128 : 256;
 }
 
 // Grouped over 128-row-aligned expert segments of A / C.
@@ -505,6 +557,10 @@ extern "C" int cm_grouped_gemm_rows_bf16(const void* A, const void* W, void* C, 
   if (rows <= 0) return 0;
   if (rows % BM) return -11;
   if ((K % 8) || (N % 8)) return -10;
+  if (pair_for_experts(rows, num_experts)) {
+    const PairArgs args{rows, N, K, expert_bn(N, b_mn != 0), N, num_experts, 0, 0, tile_expert, nullptr, err};
+    return launch_gemm_pair(PAIR_GROUPED_ROWS, false, b_mn, false, A, W, C, K, b_mn ? N : K, rows, args, stream);
+  }
   constexpr int BN = 256;
   CUtensorMap tmA, tmB;
   int rc = make_tmap_2d_bf16(&tmA, A, rows, K, K, BM);
@@ -524,6 +580,10 @@ extern "C" int cm_grouped_gemm_k_bf16(const void* A, const void* B, void* C, int
                                       cudaStream_t stream) {
   if (rows <= 0 || num_experts <= 0) return 0;
   if ((M % 8) || (N % 8)) return -10;
+  if (M > BM) {       // a pair tile needs more than one CTA's rows; with 128 or fewer its second half would be padding
+    const PairArgs args{M, N, 0, expert_bn(N, true), N, num_experts, accumulate, 0, nullptr, seg_offsets, err};
+    return launch_gemm_pair(PAIR_GROUPED_K, true, true, out_fp32, A, B, C, M, N, rows, args, stream);
+  }
   constexpr int BN = 256;
   CUtensorMap tmA, tmB;
   int rc = make_tmap_2d_bf16(&tmA, A, rows, M, M, 64);

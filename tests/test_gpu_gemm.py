@@ -107,3 +107,52 @@ def test_linear_fp32out_router_shape():
     assert rel(x.grad, xr.grad) < 2e-2
     assert rel(w.grad, wr.grad) < 2e-2
     assert w.grad.dtype == torch.float32
+
+
+@pytest.mark.parametrize("pair,bn", [(1, 256), (1, 192), (1, 128), (0, 128), (0, 64)])
+@pytest.mark.parametrize("M,N,K", [(8, 8, 8), (129, 200, 72), (257, 264, 64), (520, 776, 456), (2056, 1032, 1000)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.bfloat16, True), (torch.float32, True)])
+def test_gemm_tile_shapes(cu, pair, bn, M, N, K, a_mn, b_mn, out, accumulate):
+    """Every tile shape of the dense dispatch at sizes below, at and past the edges of its tiles, with a padded C pitch that
+    must stay untouched.  fp32 results: sums of K <= 1000 products in fp32, relative error well below 1e-5; bf16 results add
+    one rounding of 2^-9."""
+    if bn == 192 and b_mn:
+        pytest.skip("an MN-major B operand comes in runs of 64 columns per CTA")
+    torch.manual_seed(M + K)
+    M8 = (M + 7) // 8 * 8 if a_mn else M
+    A, B = torch.randn(M8, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    buf = torch.randn(M8, N + 8, device="cuda").to(out)
+    before = buf.clone()
+    a, b = (A.t().contiguous() if a_mn else A), (B.t().contiguous() if b_mn else B)
+    rc = cu.lib().cm_gemm_bf16_tiled(a.data_ptr(), b.data_ptr(), buf.data_ptr(), M8, N, K, a.stride(0), b.stride(0), buf.stride(0), int(a_mn),
+                                     int(b_mn), int(out == torch.float32), int(accumulate), pair, bn, cu.err_word(a.device).data_ptr(),
+                                     cu.stream_ptr())
+    assert rc == 0
+    cu.check_errors()
+    ref = A.double() @ B.double().t() + (before[:, :N].double() if accumulate else 0)
+    err = ((buf[:, :N].double() - ref).norm() / ref.norm()).item()
+    assert err < (1e-5 if out == torch.float32 else 4e-3)
+    assert torch.equal(buf[:, N:], before[:, N:])
+
+
+@pytest.mark.parametrize("counts", [[700, 0, 1300, 129], [5, 640, 2000, 0], [1025, 1023, 128, 896]])
+def test_grouped_experts_pair_tiles(cu, counts):
+    """Row counts for which the expert products run on CTA pairs: segments of odd and even tile counts, empty experts, and
+    widths that end inside a tile."""
+    from cppmega_b200.ops.cuda import extra
+    from cppmega_b200.ops import reference as ref
+    torch.manual_seed(4)
+    E, H, Fh = len(counts), 328, 232
+    x = torch.randn(sum(counts), H, device="cuda").bfloat16().requires_grad_()
+    w1 = (torch.randn(E, 2 * Fh, H, device="cuda") * 0.05).bfloat16().requires_grad_()
+    w2 = (torch.randn(E, H, Fh, device="cuda") * 0.05).bfloat16().requires_grad_()
+    y = extra.moe_experts(x, w1, w2, torch.tensor(counts, device="cuda"))
+    g = torch.randn_like(y)
+    y.backward(g)
+    cu.check_errors()
+    xr, w1r, w2r = (t.detach().float().requires_grad_() for t in (x, w1, w2))
+    yr = ref.grouped_gemm(ref.swiglu(ref.grouped_gemm(xr, w1r.transpose(1, 2), counts)), w2r.transpose(1, 2), counts)
+    yr.backward(g.float())
+    for got, want in ((y, yr), (x.grad, xr.grad), (w1.grad, w1r.grad), (w2.grad, w2r.grad)):
+        assert _rel(got, want) < 1.5e-2
