@@ -69,7 +69,8 @@ def _declare(L: ctypes.CDLL) -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current device's current stream, without building a ``torch.cuda.Stream`` object on every launch."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def err_word(device: Optional[torch.device] = None) -> torch.Tensor:
