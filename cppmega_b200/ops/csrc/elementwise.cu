@@ -323,96 +323,146 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_small(const __nv_bfloat16* __
   }
 }
 
-template <int TPB, int VPT>
-__device__ __forceinline__ void rms_fetch_row(uint4 (&xn)[VPT], uint4 (&gn)[VPT], float& rn, const __nv_bfloat16* __restrict__ x,
-                                              const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd_in, int row, int rows,
-                                              int H) {
-  if (row >= rows) return;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * H);
-  const uint4* gr = reinterpret_cast<const uint4*>(dy + (size_t)row * H);
-  rn = rstd_in[row];
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int idx = threadIdx.x + i * TPB;
-    if (idx < H / 8) { xn[i] = xr[idx]; gn[i] = gr[idx]; }
-  }
-}
-
-// wide rows: one CTA per row (grid-stride), dw partials for this thread's columns stay in registers
-template <int TPB, int VPT>
-__global__ void __launch_bounds__(TPB) rmsnorm_bwd_wide(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+// wide rows: one CTA works on U rows at a time (grid-stride); dw partials of this thread's columns stay in registers.  What
+// counts is the bytes in flight and the latency of a row's block-wide sum.  Every thread copies its own vectors of the next NS
+// groups of rows into shared memory with asynchronous copies and reads back only what it copied, so the copies need no
+// barrier, and the one barrier of a group (its sums alternate between two buffers) leaves them running; the U sums of a
+// group share its latency.  16,384 x 4096: 100 us (61 at the copy rate), 166 with one row per CTA
+// pass, two barriers and one row prefetched into registers.
+template <int TPB, int VPT, int U, int NS>
+__global__ void __launch_bounds__(TPB) rmsnorm_bwd_ring(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                         const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd_in,
                                                         __nv_bfloat16* __restrict__ dx, float* __restrict__ dw,
                                                         int rows, int H) {
-  __shared__ float red[TPB / 32];
-  const int nvec = H / 8;
+  extern __shared__ __align__(16) uint4 ring[];              // [NS][U][2 VPT][TPB]: slot, row, operand vector, thread
+  __shared__ float red[2][U][TPB / 32];
+  const int nvec = H / 8, tid = threadIdx.x;
+  const int groups = (rows + U - 1) / U;
   float dwacc[VPT][8];
 #pragma unroll
   for (int i = 0; i < VPT; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[i][j] = 0.f;
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
-  // the next row's vectors are requested before this row's reduction, so the block-wide sum and the two barriers
-  // of a row overlap the loads of the following one
-  uint4 xn[VPT], gn[VPT];
-  float rn = 0.f;
-  constexpr bool PREFETCH = VPT <= 4;          // wider rows would not fit two rows of operands in registers
-  if constexpr (PREFETCH) rms_fetch_row<TPB, VPT>(xn, gn, rn, x, dy, rstd_in, blockIdx.x, rows, H);
-  uint4 wv[PREFETCH ? VPT : 1];
-  if constexpr (PREFETCH) {
+  constexpr bool HOLD_W = VPT <= 2;             // wider rows read the weight again: it does not fit beside their operands
+  uint4 wv[HOLD_W ? VPT : 1];
+  auto load_w = [&](int i) {
+    const int idx = tid + i * TPB;
+    return idx < nvec ? reinterpret_cast<const uint4*>(w)[idx] : make_uint4(0, 0, 0, 0);
+  };
+  if constexpr (HOLD_W) {
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int idx = threadIdx.x + i * TPB;
-      wv[i] = idx < nvec ? wr[idx] : make_uint4(0, 0, 0, 0);
-    }
+    for (int i = 0; i < VPT; ++i) wv[i] = load_w(i);
   }
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    if constexpr (!PREFETCH) rms_fetch_row<TPB, VPT>(xn, gn, rn, x, dy, rstd_in, row, rows, H);
-    const float rstd = rn;
-    uint4 xc[VPT], gc[VPT];
+  auto copy16 = [](uint4* dst, const uint4* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+  };
+  auto at = [&](int slot, int u, int i, int op) { return ring + (((slot * U + u) * VPT + i) * 2 + op) * TPB + tid; };
+  auto request = [&](int grp, int slot) {       // one commit per group of rows, empty past the last
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) { xc[i] = xn[i]; gc[i] = gn[i]; }
-    if constexpr (PREFETCH) rms_fetch_row<TPB, VPT>(xn, gn, rn, x, dy, rstd_in, row + gridDim.x, rows, H);
-    float xh[VPT][8], gw[VPT][8];
-    float dot = 0.f;
+    for (int u = 0; u < U; ++u) {
+      const int row = grp * U + u;
+      if (grp < groups && row < rows) {
+        const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * H);
+        const uint4* gr = reinterpret_cast<const uint4*>(dy + (size_t)row * H);
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int idx = threadIdx.x + i * TPB;
-      if (idx < nvec) {
-        const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&xc[i]);
-        const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gc[i]);
-        uint4 wcur;
-        if constexpr (PREFETCH) wcur = wv[i]; else wcur = wr[idx];
-        const __nv_bfloat162* wb = reinterpret_cast<const __nv_bfloat162*>(&wcur);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float2 xf = __bfloat1622float2(xb[j]), gf = __bfloat1622float2(gb[j]), wf = __bfloat1622float2(wb[j]);
-          xh[i][2 * j] = xf.x * rstd;       xh[i][2 * j + 1] = xf.y * rstd;
-          gw[i][2 * j] = gf.x * wf.x;       gw[i][2 * j + 1] = gf.y * wf.y;
-          dwacc[i][2 * j] += gf.x * xh[i][2 * j];
-          dwacc[i][2 * j + 1] += gf.y * xh[i][2 * j + 1];
-          dot += gw[i][2 * j] * xh[i][2 * j] + gw[i][2 * j + 1] * xh[i][2 * j + 1];
+        for (int i = 0; i < VPT; ++i) {
+          const int idx = tid + i * TPB;
+          if (idx < nvec) {
+            copy16(at(slot, u, i, 0), xr + idx);
+            copy16(at(slot, u, i, 1), gr + idx);
+          }
         }
       }
     }
-    dot = warp_sum(dot);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dot;
-    __syncthreads();
-    float tot = 0.f;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float rs_next[U];
+  auto load_rstd = [&](int grp) {
 #pragma unroll
-    for (int i = 0; i < TPB / 32; ++i) tot += red[i];
-    __syncthreads();
-    dot = tot / H;
-    uint4* dxr = reinterpret_cast<uint4*>(dx + (size_t)row * H);
+    for (int u = 0; u < U; ++u) rs_next[u] = grp < groups && grp * U + u < rows ? rstd_in[grp * U + u] : 0.f;
+  };
+  for (int s = 0; s < NS; ++s) request(blockIdx.x + s * gridDim.x, s);
+  load_rstd(blockIdx.x);
+  int slot = 0, buf = 0;
+  for (int grp = blockIdx.x; grp < groups; grp += gridDim.x, buf ^= 1) {
+    float rs[U], dot[U];
+    uint4 xv[U][VPT], gv[U][VPT];
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) {
-      const int idx = threadIdx.x + i * TPB;
-      if (idx < nvec) {
+    for (int u = 0; u < U; ++u) rs[u] = rs_next[u];
+    load_rstd(grp + gridDim.x);
+    asm volatile("cp.async.wait_group %0;" ::"n"(NS - 1) : "memory");
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const bool on = tid + i * TPB < nvec && grp * U + u < rows;
+        xv[u][i] = on ? *at(slot, u, i, 0) : make_uint4(0, 0, 0, 0);
+        gv[u][i] = on ? *at(slot, u, i, 1) : make_uint4(0, 0, 0, 0);
+      }
+    request(grp + NS * gridDim.x, slot);
+    if (++slot == NS) slot = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      dot[u] = 0.f;
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        uint4 wc;
+        if constexpr (HOLD_W) wc = wv[i]; else wc = load_w(i);
+        const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&xv[u][i]);
+        const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gv[u][i]);
+        const __nv_bfloat162* wb = reinterpret_cast<const __nv_bfloat162*>(&wc);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 xf = __bfloat1622float2(xb[j]), gf = __bfloat1622float2(gb[j]), wf = __bfloat1622float2(wb[j]);
+          const float h0 = xf.x * rs[u], h1 = xf.y * rs[u];
+          dwacc[i][2 * j] += gf.x * h0;
+          dwacc[i][2 * j + 1] += gf.y * h1;
+          dot[u] += gf.x * wf.x * h0 + gf.y * wf.y * h1;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < U; ++u) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
+    if ((tid & 31) == 0) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) red[buf][u][tid >> 5] = dot[u];
+    }
+    __syncthreads();
+    // the packed operands are unpacked again below: held as floats over the barrier they would take four times the registers
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        asm volatile("" : "+r"(xv[u][i].x), "+r"(xv[u][i].y), "+r"(xv[u][i].z), "+r"(xv[u][i].w));
+        asm volatile("" : "+r"(gv[u][i].x), "+r"(gv[u][i].y), "+r"(gv[u][i].z), "+r"(gv[u][i].w));
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int row = grp * U + u;
+      if (row >= rows) break;
+      float tot = 0.f;
+#pragma unroll
+      for (int i = 0; i < TPB / 32; ++i) tot += red[buf][u][i];
+      tot /= H;
+      uint4* dxr = reinterpret_cast<uint4*>(dx + (size_t)row * H);
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) {
+        const int idx = tid + i * TPB;
+        if (idx >= nvec) continue;
+        uint4 wc;
+        if constexpr (HOLD_W) wc = wv[i]; else wc = load_w(i);
+        const __nv_bfloat162* xb = reinterpret_cast<const __nv_bfloat162*>(&xv[u][i]);
+        const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gv[u][i]);
+        const __nv_bfloat162* wb = reinterpret_cast<const __nv_bfloat162*>(&wc);
         uint4 o;
         uint32_t* op = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          op[j] = pack_bf16(rstd * (gw[i][2 * j] - xh[i][2 * j] * dot), rstd * (gw[i][2 * j + 1] - xh[i][2 * j + 1] * dot));
+        for (int j = 0; j < 4; ++j) {
+          const float2 xf = __bfloat1622float2(xb[j]), gf = __bfloat1622float2(gb[j]), wf = __bfloat1622float2(wb[j]);
+          op[j] = pack_bf16(rs[u] * (gf.x * wf.x - xf.x * rs[u] * tot), rs[u] * (gf.y * wf.y - xf.y * rs[u] * tot));
+        }
         dxr[idx] = o;
       }
     }
@@ -420,7 +470,7 @@ __global__ void __launch_bounds__(TPB) rmsnorm_bwd_wide(const __nv_bfloat16* __r
   if (dw) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      const int idx = threadIdx.x + i * TPB;
+      const int idx = tid + i * TPB;
       if (idx < nvec) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) atomicAdd(dw + idx * 8 + j, dwacc[i][j]);
@@ -714,6 +764,20 @@ extern "C" int cm_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+template <int TPB, int VPT, int U, int NS>
+static int launch_rmsnorm_ring(const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* dy, const float* rstd, __nv_bfloat16* dx,
+                               float* dw, int rows, int H, int per_sm, cudaStream_t s) {
+  constexpr int SMEM = NS * U * 2 * VPT * TPB * 16;
+  static PerDevice cfg;
+  if (cfg.first()) {
+    if (cudaFuncSetAttribute(rmsnorm_bwd_ring<TPB, VPT, U, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) return -2;
+    cfg.done();
+  }
+  const int cap = sm_count() * per_sm, groups = (rows + U - 1) / U;
+  rmsnorm_bwd_ring<TPB, VPT, U, NS><<<groups < cap ? groups : cap, TPB, SMEM, s>>>(x, w, dy, rstd, dx, dw, rows, H);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
 extern "C" int cm_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, void* dx, float* dw,
                               int rows, int H, cudaStream_t s) {
   if (rows <= 0) return 0;
@@ -730,9 +794,14 @@ extern "C" int cm_rmsnorm_bwd(const void* x, const void* w, const void* dy, cons
   else if (H == 128) rmsnorm_bwd_small<16><<<small_grid(2), 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows);
   else if (H == 256) rmsnorm_bwd_small<32><<<small_grid(1), 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows);
   else if (H <= 32 * 1 * 8) rmsnorm_bwd_kernel<1><<<grid, 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows, H);
-  else if (H <= 128 * 1 * 8) rmsnorm_bwd_wide<128, 1><<<(rows < cap ? rows : cap), 128, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows, H);
-  else if (H <= 256 * 2 * 8) rmsnorm_bwd_wide<256, 2><<<(rows < cap ? rows : cap), 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows, H);
-  else if (H <= 256 * 8 * 8) rmsnorm_bwd_wide<256, 8><<<(rows < cap ? rows : cap), 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows, H);
+  // rings of 32, 64 and 192 KB: 6, 3 and 1 CTAs per SM; calls of few rows take one row to a CTA
+  else if (H <= 128 * 1 * 8) {
+    if (rows >= sm_count() * 6 * 4) return launch_rmsnorm_ring<128, 1, 2, 4>(xp, wp, gp, rstd, dxp, dw, rows, H, 6, s);
+    return launch_rmsnorm_ring<128, 1, 1, 2>(xp, wp, gp, rstd, dxp, dw, rows, H, 6, s);
+  } else if (H <= 256 * 2 * 8) {
+    if (rows >= sm_count() * 3 * 2) return launch_rmsnorm_ring<256, 2, 2, 2>(xp, wp, gp, rstd, dxp, dw, rows, H, 3, s);
+    return launch_rmsnorm_ring<256, 2, 1, 2>(xp, wp, gp, rstd, dxp, dw, rows, H, 3, s);
+  } else if (H <= 256 * 8 * 8) return launch_rmsnorm_ring<256, 8, 1, 3>(xp, wp, gp, rstd, dxp, dw, rows, H, 1, s);
   else return -12;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -26,6 +26,25 @@ def test_rmsnorm(rows, H):
     assert _rel(w.grad, wr.grad) < 8e-3
 
 
+@pytest.mark.parametrize("H", [264, 816, 1024, 1032, 3584, 4096, 4104])
+@pytest.mark.parametrize("rows", [1, 297, 887, 889, 1187, 3553, 5003])
+def test_rmsnorm_backward_row_groups(rows, H):
+    """Row counts on both sides of the thresholds at which a CTA takes two rows at a time (888 and 3552 on 148 SMs), with
+    remainders and with fewer and more groups than ring slots, at widths that fill the thread block and that do not.  One bf16 rounding of each result: 2^-9 relative at
+    most, 1.7e-3 in the mean; dw is summed in fp32 first."""
+    from cppmega_b200.ops import cuda as cu, reference as ref
+    torch.manual_seed(rows + H)
+    x = torch.randn(rows, H, device="cuda").bfloat16().requires_grad_()
+    w = (1 + 0.1 * torch.randn(H, device="cuda")).bfloat16().requires_grad_()
+    y = cu.rmsnorm(x, w, 1e-5)
+    g = torch.randn_like(y)
+    y.backward(g)
+    xr, wr = x.detach().float().requires_grad_(), w.detach().float().requires_grad_()
+    ref.rmsnorm(xr, wr, 1e-5).backward(g.float())
+    assert _rel(x.grad, xr.grad) < 4e-3
+    assert _rel(w.grad, wr.grad) < 4e-3
+
+
 @pytest.mark.parametrize("n", [8, 8 * 1023, 8 * 512 * 148 * 8 + 8])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_scale_to_bf16(n, dtype):
