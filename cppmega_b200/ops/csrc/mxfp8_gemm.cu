@@ -20,12 +20,16 @@
 // stacked [E*N, K] weights) or b_k_e columns further right (dgrad: the stacked transposed weights [N, E*K]);
 // GROUPED_K reduces over per-expert ranges of the shared K axis (token rows, multiples of 128) into a stack [E, M, N]
 // (expert weight gradients from the token-transposed operands).
+// Dense problems that fill the chip with 256-row tiles run on CTA pairs (mxfp8_pair_kernel): tcgen05.mma.cta_group::2 on a
+// 256 x 256 tile, each CTA with its 128 rows of A and half of B.  At 128 x 256 a CTA's shared memory takes 48 KB from TMA and
+// gives 48 KB to the tensor core per 512-cycle k tile, 192 bytes a cycle against the 128 it has; the pair needs 128.
+// The three products of an 8192 x 8192 x 4096 linear: 709 -> 560 us (2.95 PFLOP/s).
 // The other products of a linear layer use the same kernel on operands quantised along their own reduction
 // dimension and stored transposed (dgrad: dy along N with W^T; wgrad: dy^T and x^T along tokens), so no
 // MN-major FP8 path is needed.  This is the sm_100 counterpart of the reference's CUTLASS / FlashInfer MXFP8 GEMM
 // wrappers (cppmega/megatron/cutlass_mxfp8_gemm.py:102-506, cppmega/megatron/flashinfer_mxfp8_gemm.py:146-160,
 // cuda_ext/cutlass_mxfp8_gemm.cu:56-360).
-#include "common.cuh"
+#include "gemm_pair.cuh"
 
 namespace cm {
 namespace mxg {
@@ -92,6 +96,66 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)),
                "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
+}
+
+// 128 accumulator columns of one row: C[row, col0 ..] (+)= r, of output `e` of a stack
+template <typename OutT, bool ACC>
+__device__ __forceinline__ void store_rows(OutT* __restrict__ C, const Args& args, const uint32_t (&r)[4][32], int row, int col0, int e) {
+  if (row >= args.M || col0 >= args.N) return;
+  OutT* crow = C + (long long)e * args.M * args.ldc + (long long)row * args.ldc + col0;
+  if (col0 + 128 <= args.N && (args.ldc % 8) == 0) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if constexpr (sizeof(OutT) == 2) {
+        uint4* dst = reinterpret_cast<uint4*>(crow + c * 32);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          float f[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[c][v * 8 + j]);
+          if (ACC) {
+            const uint4 old = dst[v];
+            const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 t = __bfloat1622float2(ob[j]);
+              f[2 * j] += t.x; f[2 * j + 1] += t.y;
+            }
+          }
+          uint4 o;
+          o.x = pack_bf16(f[0], f[1]);
+          o.y = pack_bf16(f[2], f[3]);
+          o.z = pack_bf16(f[4], f[5]);
+          o.w = pack_bf16(f[6], f[7]);
+          dst[v] = o;
+        }
+      } else {
+        float4* dst = reinterpret_cast<float4*>(crow + c * 32);
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          float4 o = make_float4(__uint_as_float(r[c][v * 4 + 0]), __uint_as_float(r[c][v * 4 + 1]),
+                                 __uint_as_float(r[c][v * 4 + 2]), __uint_as_float(r[c][v * 4 + 3]));
+          if (ACC) {
+            const float4 old = dst[v];
+            o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+          }
+          dst[v] = o;
+        }
+      }
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        if (col0 + c * 32 + j < args.N) {
+          float v = __uint_as_float(r[c][j]);
+          if (ACC) v += float(crow[c * 32 + j]);
+          crow[c * 32 + j] = OutT(v);
+        }
+      }
+    }
+  }
 }
 
 template <typename OutT, bool ACC, int MODE>
@@ -267,63 +331,7 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(tmem_empty);   // the accumulator is in registers: the next tile may start
 
-      const int row = mt * BM + q * 32 + lane;
-      const int col0 = nt * BN + half * 128;
-      if (row >= args.M || col0 >= args.N) continue;
-      OutT* crow = C + (MODE == GROUPED_K ? (long long)t.e * args.M * args.ldc : 0ll) + (long long)row * args.ldc + col0;
-      if (col0 + 128 <= args.N && (args.ldc % 8) == 0) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if constexpr (sizeof(OutT) == 2) {
-            uint4* dst = reinterpret_cast<uint4*>(crow + c * 32);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              float f[8];
-#pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[c][v * 8 + j]);
-              if (ACC) {
-                const uint4 old = dst[v];
-                const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&old);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float2 t = __bfloat1622float2(ob[j]);
-                  f[2 * j] += t.x; f[2 * j + 1] += t.y;
-                }
-              }
-              uint4 o;
-              o.x = pack_bf16(f[0], f[1]);
-              o.y = pack_bf16(f[2], f[3]);
-              o.z = pack_bf16(f[4], f[5]);
-              o.w = pack_bf16(f[6], f[7]);
-              dst[v] = o;
-            }
-          } else {
-            float4* dst = reinterpret_cast<float4*>(crow + c * 32);
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-              float4 o = make_float4(__uint_as_float(r[c][v * 4 + 0]), __uint_as_float(r[c][v * 4 + 1]),
-                                     __uint_as_float(r[c][v * 4 + 2]), __uint_as_float(r[c][v * 4 + 3]));
-              if (ACC) {
-                const float4 old = dst[v];
-                o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-              }
-              dst[v] = o;
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (col0 + c * 32 + j < args.N) {
-              float v = __uint_as_float(r[c][j]);
-              if (ACC) v += float(crow[c * 32 + j]);
-              crow[c * 32 + j] = OutT(v);
-            }
-          }
-        }
-      }
+      store_rows<OutT, ACC>(C, args, r, mt * BM + q * 32 + lane, nt * BN + half * 128, MODE == GROUPED_K ? t.e : 0);
     }
   }
 
@@ -339,6 +347,191 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// CTA pairs, dense.  Barriers and roles as in gemm_pair.cu; epilogue warps as above.  The scale tiles come through tensor
+// maps too (rows of 128 words), since only those loads may signal the first CTA's barrier from the second.  Each CTA holds the
+// scales of its own 128 rows of A and of all 256 rows of B; they alternate between two sets of TMEM columns, so that the
+// copies for a k tile do not wait for the products of the one before.
+// ------------------------------------------------------------------------------------------
+namespace mxpair {
+constexpr int STAGES = 6;
+constexpr int OP_BYTES = 128 * BK;                              // one CTA's rows of A, or of B, per stage
+constexpr int SF_BYTES = 512 + 1024;
+constexpr int SF_OFF = STAGES * 2 * OP_BYTES;
+constexpr int BAR_OFF = SF_OFF + STAGES * SF_BYTES;
+constexpr int SMEM_TOTAL = BAR_OFF + 256 + 1024;
+constexpr int SF_COLS = 16;
+
+__device__ __forceinline__ void cp_sf(uint32_t taddr, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+__device__ __forceinline__ void mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                    uint32_t accumulate) {
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n"
+      "}\n" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
+      : "memory");
+}
+}  // namespace mxpair
+
+template <typename OutT, bool ACC>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmSA,
+                  const __grid_constant__ CUtensorMap tmSB, OutT* __restrict__ C, const Args args) {
+  using namespace pair2;
+  namespace mp = mxpair;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + mp::STAGES * mp::OP_BYTES;
+  uint8_t* sSF = smem + mp::SF_OFF;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + mp::BAR_OFF);
+  uint64_t* empty_bar = full_bar + mp::STAGES;
+  uint64_t* tmem_full = empty_bar + mp::STAGES;
+  uint64_t* tmem_empty = tmem_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const int first_tile = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  const int tiles_n = (args.N + BN - 1) / BN, tiles_m = (args.M + 2 * BM - 1) / (2 * BM), total = tiles_m * tiles_n;
+  const int nkt = (args.K + BK - 1) / BK;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < mp::STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(tmem_full, 1);
+    mbar_init(tmem_empty, 16);
+    *abort_flag = (args.err && *reinterpret_cast<volatile int*>(args.err) != 0) ? 1 : 0;   // an earlier kernel gave up: drain
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  auto decode = [&](int tile, int& mt, int& nt) {               // bands of 8 row tiles share B tiles in L2
+    const int band_tiles = 8 * tiles_n, b = tile / band_tiles, in = tile - b * band_tiles;
+    const int rows = min(8, tiles_m - b * 8);
+    mt = b * 8 + in % rows;
+    nt = in / rows;
+  };
+
+  if (warp == 0) {
+    if (elect_one()) {
+      tma_prefetch_desc(&tmA);
+      tma_prefetch_desc(&tmB);
+      uint32_t stage = 0, phase = 0, used = 0;
+      bool ok = *abort_flag == 0;
+      for (int tile = first_tile; tile < total && ok; tile += tile_step) {
+        int mt, nt;
+        decode(tile, mt, nt);
+        const bool two = nt * BN + 128 < args.N;                // the second 128-row scale tile of B exists
+        const uint32_t pair_bytes = 2 * (2 * mp::OP_BYTES + 512 + (two ? 1024 : 512));
+        for (int kt = 0; kt < nkt; ++kt) {
+          ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, args.err, ERR_WAIT_EMPTY);
+          if (!ok) break;
+          if (rank == 0) mbar_expect_tx(&full_bar[stage], pair_bytes);
+          const uint32_t bar = map_to_rank(smem_u32(&full_bar[stage]), 0);
+          uint8_t* sf = sSF + stage * mp::SF_BYTES;
+          load_2d(sA + stage * mp::OP_BYTES, &tmA, bar, kt * BK, mt * 2 * BM + rank * BM);
+          load_2d(sB + stage * mp::OP_BYTES, &tmB, bar, kt * BK, nt * BN + rank * 128);
+          load_2d(sf, &tmSA, bar, 0, (mt * 2 + rank) * args.sfa_nkt + kt);
+          load_2d(sf + 512, &tmSB, bar, 0, nt * 2 * args.sfb_nkt + kt);
+          if (two) load_2d(sf + 1024, &tmSB, bar, 0, (nt * 2 + 1) * args.sfb_nkt + kt);
+          if (used < mp::STAGES) ++used;
+          if (++stage == mp::STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+      // the last releases of this CTA's stages come from the partner: see them arrive before the barriers go away
+      for (uint32_t i = 0; i < used && ok; ++i) {
+        const uint32_t s = (stage + mp::STAGES - 1 - i) % mp::STAGES;
+        ok = mbar_wait(&empty_bar[s], stage >= i + 1 ? phase : phase ^ 1, abort_flag, args.err, ERR_WAIT_EMPTY);
+      }
+    }
+  } else if (warp == 1) {
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc0 = idesc_mxf8(2 * BM, BN);
+      uint32_t stage = 0, phase = 0, acc_phase = 0, set = 0;
+      bool ok = *abort_flag == 0;
+      for (int tile = first_tile; tile < total && ok; tile += tile_step) {
+        int mt, nt;
+        decode(tile, mt, nt);
+        const bool two = nt * BN + 128 < args.N;
+        ok = mbar_wait(tmem_empty, acc_phase ^ 1, abort_flag, args.err, ERR_WAIT_TMEM_EMPTY);
+        if (!ok) break;
+        tc_fence_after();
+        for (int kt = 0; kt < nkt; ++kt) {
+          ok = mbar_wait(&full_bar[stage], phase, abort_flag, args.err, ERR_WAIT_FULL);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t sa = smem_u32(sA + stage * mp::OP_BYTES), sb = smem_u32(sB + stage * mp::OP_BYTES);
+          const uint32_t sf = smem_u32(sSF + stage * mp::SF_BYTES);
+          const uint32_t sfa = tmem_base + 256 + set * mp::SF_COLS, sfb = sfa + 4;
+          set ^= 1;
+          mp::cp_sf(sfa, sf_desc(sf));
+          mp::cp_sf(sfb, sf_desc(sf + 512));
+          if (two) mp::cp_sf(sfb + 4, sf_desc(sf + 1024));
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            mp::mma(tmem_base, umma_desc_sw128(sa + k * 32, 16, 1024), umma_desc_sw128(sb + k * 32, 16, 1024),
+                    idesc0 | (uint32_t(k) << 29) | (uint32_t(k) << 4), sfa, sfb, (kt | k) != 0);
+          commit_pair(&empty_bar[stage]);
+          if (++stage == mp::STAGES) { stage = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+        commit_pair(tmem_full);
+        acc_phase ^= 1;
+      }
+    }
+  } else {
+    const int q = warp & 3;                    // TMEM lane quarter this warp may read
+    const int half = (warp - 2) >> 2;          // which 128 of the 256 accumulator columns
+    uint32_t acc_phase = 0;
+    bool ok = *abort_flag == 0;
+    for (int tile = first_tile; tile < total && ok; tile += tile_step) {
+      int mt, nt;
+      decode(tile, mt, nt);
+      ok = __all_sync(0xffffffffu, mbar_wait(tmem_full, acc_phase, abort_flag, args.err, ERR_WAIT_TMEM_FULL));
+      if (!ok) break;
+      acc_phase ^= 1;
+      tc_fence_after();
+      uint32_t r[4][32];
+      const uint32_t t_base = tmem_base + half * 128 + (uint32_t(q * 32) << 16);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(t_base + c * 32, r[c]);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_to_rank(smem_u32(tmem_empty), 0));   // in registers: the next tile may start
+      store_rows<OutT, ACC>(C, args, r, mt * 2 * BM + (int)rank * BM + q * 32 + lane, nt * BN + half * 128, 0);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);      // let copies still in flight land before the pair goes away
+    __syncthreads();
+  }
+  cluster_sync();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+  }
+}
+
 static int make_tmap_u8(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return -1;
@@ -349,6 +542,37 @@ static int make_tmap_u8(CUtensorMap* out, const void* base, uint64_t rows, uint6
   CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : int(r);
+}
+
+// Scale tiles as rows of 128 words
+static int make_tmap_sf(CUtensorMap* out, const void* base, uint64_t tiles) {
+  EncodeTiledFn enc = get_encode_tiled();
+  if (!enc) return -1;
+  cuuint64_t dims[2] = {128, tiles};
+  cuuint64_t strides[1] = {512};
+  cuuint32_t box[2] = {128, 1};
+  cuuint32_t es[2] = {1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : int(r);
+}
+
+template <typename OutT, bool ACC>
+static int launch_pair(const void* A, const void* B, void* C, long long lda, long long ldb, const Args& args, int tiles, cudaStream_t s) {
+  CUtensorMap tmA, tmB, tmSA, tmSB;
+  if (int rc = make_tmap_u8(&tmA, A, args.M, args.K, lda, BM)) return 100 + rc;
+  if (int rc = make_tmap_u8(&tmB, B, args.N, args.K, ldb, 128)) return 100 + rc;
+  if (int rc = make_tmap_sf(&tmSA, args.sfa, (uint64_t)((args.M + 127) / 128) * args.sfa_nkt)) return 100 + rc;
+  if (int rc = make_tmap_sf(&tmSB, args.sfb, (uint64_t)((args.N + 127) / 128) * args.sfb_nkt)) return 100 + rc;
+  auto kern = mxfp8_pair_kernel<OutT, ACC>;
+  static PerDevice attr_set;
+  if (attr_set.first()) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, mxpair::SMEM_TOTAL) != cudaSuccess) return -2;
+    attr_set.done();
+  }
+  const int pairs = sm_count() / 2;
+  kern<<<2 * (tiles < pairs ? tiles : pairs), THREADS, mxpair::SMEM_TOTAL, s>>>(tmA, tmB, tmSA, tmSB, reinterpret_cast<OutT*>(C), args);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
 template <typename OutT, bool ACC, int MODE = DENSE>
@@ -384,6 +608,15 @@ extern "C" int cm_mxfp8_gemm(const void* A, const void* sfa, const void* B, cons
   if (int rc = make_tmap_u8(&tmB, B, N, K, ldb, BN)) return 100 + rc;
   const int nkt = (K + BK - 1) / BK;
   Args args{M, N, K, ldc, (const uint8_t*)sfa, (const uint8_t*)sfb, err, nkt, nkt, nullptr, nullptr, 1, 0, 0};
+  // a wave of pair tiles and a wave of one-CTA tiles cover the same area: pairs wherever they need no more waves
+  const int tn = (N + BN - 1) / BN, pair_tiles = (M + 255) / 256 * tn, one_tiles = (M + 127) / 128 * tn, sms = sm_count();
+  if (M > BM && (pair_tiles + sms / 2 - 1) / (sms / 2) <= (one_tiles + sms - 1) / sms) {
+    if (!out_fp32)
+      return accumulate ? launch_pair<__nv_bfloat16, true>(A, B, C, lda, ldb, args, pair_tiles, s)
+                        : launch_pair<__nv_bfloat16, false>(A, B, C, lda, ldb, args, pair_tiles, s);
+    return accumulate ? launch_pair<float, true>(A, B, C, lda, ldb, args, pair_tiles, s)
+                      : launch_pair<float, false>(A, B, C, lda, ldb, args, pair_tiles, s);
+  }
   if (!out_fp32) return accumulate ? launch<__nv_bfloat16, true>(tmA, tmB, C, args, s) : launch<__nv_bfloat16, false>(tmA, tmB, C, args, s);
   return accumulate ? launch<float, true>(tmA, tmB, C, args, s) : launch<float, false>(tmA, tmB, C, args, s);
 }

@@ -524,3 +524,22 @@ def test_mxfp8_quantize_both_tile_edges(rows, cols):
         pay, sc = (pay, sc) if axis == 1 else (pay.t(), sc.t())
         assert torch.equal(got.scales, sc.contiguous())
         assert torch.equal(got.payload, pay.contiguous().view(torch.uint8))
+
+@pytest.mark.parametrize("M,N,K", [(160, 96, 64), (256, 256, 128), (288, 416, 1056), (2080, 4128, 416), (4128, 9504, 160)])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.bfloat16, True), (torch.float32, True)])
+def test_mxfp8_gemm_pair_tiles(M, N, K, out, accumulate):
+    """Sizes that end inside the 256 x 256 x 128 tiles of the CTA-pair kernel: a missing second row tile, one scale tile of B
+    instead of two, a last k tile of 32.  The reference multiplies the dequantised operands in 64 bits: fp32 results differ by
+    the summation (below 1e-5), bf16 results by one rounding."""
+    from cppmega_b200.ops import cuda as cu
+    from cppmega_b200.ops.cuda import mxfp8
+    torch.manual_seed(M + K)
+    spread = lambda r: torch.exp2(torch.randint(-4, 4, (r, 1), device="cuda").float())  # noqa: E731
+    a = mxfp8.quantize_rowwise((torch.randn(M, K, device="cuda") * spread(M)).bfloat16())
+    b = mxfp8.quantize_rowwise((torch.randn(N, K, device="cuda") * spread(N)).bfloat16())
+    c0 = torch.randn(M, N, device="cuda").to(out)
+    c = mxfp8.gemm_mxfp8(a, b, out=c0.clone(), accumulate=accumulate)
+    cu.check_errors()
+    # an E4M3 value times a power of two is exact in bf16
+    want = mxfp8.dequantize(a).double() @ mxfp8.dequantize(b).double().t() + (c0.double() if accumulate else 0)
+    assert ((c.double() - want).norm() / want.norm()).item() < (1e-5 if out == torch.float32 else 4e-3)
