@@ -201,14 +201,13 @@ __global__ void __launch_bounds__(256) angle_reduce_kernel(const float* __restri
 // Per-head operand gradients of the scan -> gradients of the group-shared operand and of the per-head bias:
 //   dgrp[t, g, c]  = sum_{h in group g} dh[t, h, c]            (bf16 out)
 //   dbias[h, c]   += sum_t dh[t, h, c]                          (fp32, atomically accumulated; caller zeroes)
-// dh [T, H, C] bf16 with C = R * N columns.  One block covers TT tokens of one group; a thread owns two columns.
-constexpr int HR_TT = 64;
+// dh [T, H, C] bf16 with C = R * N columns.  One block covers `tt` tokens of one group; a thread owns two columns.
 template <int HPG>
 __global__ void __launch_bounds__(256) head_reduce_kernel(const __nv_bfloat16* __restrict__ dh, __nv_bfloat16* __restrict__ dgrp,
-                                                          float* __restrict__ dbias, long long T, int H, int C) {
+                                                          float* __restrict__ dbias, long long T, int H, int C, int tt) {
   const int g = blockIdx.y, G = H / HPG;
-  const long long t0 = (long long)blockIdx.x * HR_TT;
-  const long long t1 = t0 + HR_TT < T ? t0 + HR_TT : T;
+  const long long t0 = (long long)blockIdx.x * tt;
+  const long long t1 = t0 + tt < T ? t0 + tt : T;
   for (int c2 = threadIdx.x; c2 < C / 2; c2 += blockDim.x) {
     float bx[HPG], by[HPG];
 #pragma unroll
@@ -240,15 +239,19 @@ using namespace cm;
 extern "C" int cm_head_reduce(const void* dh, void* dgrp, float* dbias, long long T, int H, int G, int C, cudaStream_t s) {
   if (T <= 0) return 0;
   if (C % 2 || H % G) return -10;
-  dim3 grid((unsigned)((T + HR_TT - 1) / HR_TT), G);
+  // 64 tokens a block keep the bias atomics rare; a call too small to give every SM two such blocks is cut finer, since the
+  // tokens of a block are walked one after the other (512 tokens, one group: 37 us with 8 blocks, 7 with 64)
+  int tt = 64;
+  while (tt > 8 && (T + tt - 1) / tt * G < 2ll * sm_count()) tt >>= 1;
+  dim3 grid((unsigned)((T + tt - 1) / tt), G);
   const int hpg = H / G;
   auto a = (const __nv_bfloat16*)dh;
   auto o = (__nv_bfloat16*)dgrp;
-  if (hpg == 16) head_reduce_kernel<16><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C);
-  else if (hpg == 8) head_reduce_kernel<8><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C);
-  else if (hpg == 4) head_reduce_kernel<4><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C);
-  else if (hpg == 2) head_reduce_kernel<2><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C);
-  else if (hpg == 1) head_reduce_kernel<1><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C);
+  if (hpg == 16) head_reduce_kernel<16><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C, tt);
+  else if (hpg == 8) head_reduce_kernel<8><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C, tt);
+  else if (hpg == 4) head_reduce_kernel<4><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C, tt);
+  else if (hpg == 2) head_reduce_kernel<2><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C, tt);
+  else if (hpg == 1) head_reduce_kernel<1><<<grid, 256, 0, s>>>(a, o, dbias, T, H, C, tt);
   else return -12;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -55,6 +55,8 @@ struct BwdArgs {
   float* dZeta;
   float* dPhi;
   float* dD;                    // [H]
+  float* dQb;                   // [H,R,N] sums over tokens of dQh / dKh (may be null); zeroed by grad_state like the four above
+  float* dKb;
   int B, S, H, G, C;
   long long ldV, ldZ;           // token strides of V and Z in elements
   int* err;
@@ -123,6 +125,17 @@ __global__ void __launch_bounds__(THREADS2) mimo_grad_state_kernel(const __grid_
   decode_block_b(a, b, g, c, h);
   const int t0 = c * LT;
   const int i = threadIdx.x & 127, wg = threadIdx.x >> 7, t = i >> 2, r = i & 3, warp = threadIdx.x >> 5;
+  if (b == 0 && c == 0) {                          // the accumulators of head h that later kernels add to
+    static_assert(R * P == THREADS2 && R * N == 2 * THREADS2, "one element of each [R,P] vector per thread");
+    a.dPsi[h * R * P + threadIdx.x] = 0.f;
+    a.dZeta[h * R * P + threadIdx.x] = 0.f;
+    a.dPhi[h * R * P + threadIdx.x] = 0.f;
+    if (threadIdx.x == 0) a.dD[h] = 0.f;
+    if (a.dQb) {
+      reinterpret_cast<float2*>(a.dQb + (size_t)h * R * N)[threadIdx.x] = make_float2(0.f, 0.f);
+      reinterpret_cast<float2*>(a.dKb + (size_t)h * R * N)[threadIdx.x] = make_float2(0.f, 0.f);
+    }
+  }
   // every global load of the prologue is issued here, ahead of the set-up, and consumed further down
   const ScalarLoads sl = load_chunk_scalars(a.ADT, a.DT, a.Trap, ((size_t)b * a.H + h) * a.S + t0, t0, a.S);
   const float4 ang4 = load_angles4<NROT>(a.angles, b, t0, h, a.S, a.H);
@@ -729,6 +742,19 @@ __global__ void __launch_bounds__(THREADS2, 1) mimo_chunk_grad_kernel(const __gr
   if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
+// Trapezoid coefficients: gamma_t = DT_t sig(Trap_t), ts_t = gamma_t + DT_{t+1} sig(-Trap_{t+1}); their gradients to DT, Trap.
+// One launch instead of the dozen elementwise launches of the tensor library that cost a small call more than its kernels.
+__global__ void __launch_bounds__(256) mimo_trapezoid_grad_kernel(const float* __restrict__ dts, const float* __restrict__ dgam,
+                                                                  const float* __restrict__ DT, const float* __restrict__ Trap,
+                                                                  float* __restrict__ dDT, float* __restrict__ dTrap, long long n, int S) {
+  for (long long x = blockIdx.x * 256ll + threadIdx.x; x < n; x += gridDim.x * 256ll) {
+    const float sg = 1.f / (1.f + expf(-Trap[x]));
+    const float dgt = dgam[x] + dts[x], prev = x % S ? dts[x - 1] : 0.f;
+    dDT[x] = dgt * sg + prev * (1.f - sg);
+    dTrap[x] = (dgt - prev) * DT[x] * sg * (1.f - sg);
+  }
+}
+
 constexpr int grad_state_smem() {
   return 2 * SLAB + SLAB + 2 * tab_floats<32>() * 4 + (int)sizeof(HeadBias<128>) + (int)sizeof(HeadVecs) + (int)sizeof(ChunkScalars) + 64 + 1024;
 }
@@ -745,14 +771,17 @@ using namespace cm::mimo;
 // Inputs as in cm_mimo_scan_fwd plus dY [B,S,H,P] bf16, the forward's `states` (start states, bf16) and `tot`.
 // Scratch: gbuf [B,H,C,N,P] fp32, dend [B,H,C,N,P] bf16.
 // Outputs: dQh, dKh [B,S,H,R,N] bf16 (per head, before the group reduction); dV, dZ [B,S,H,P] bf16;
-// dAngles [B,S,H,N/4] fp32; dADT, dTs, dGam [B,H,S] fp32; dPsi, dZeta, dPhi [H,R,P], dD [H] fp32 (accumulated:
-// the caller zeroes them).
+// dAngles [B,S,H,N/4] fp32; dADT, dTs, dGam [B,H,S] fp32; dPsi, dZeta, dPhi [H,R,P], dD [H] fp32;
+// dDT, dTrap [B,H,S] fp32.  dQg, dKg [B,S,G,R,N] bf16 and dQb, dKb [H,R,N] fp32 (all or none; H / G in 1, 2, 4, 8, 16): the
+// sums of dQh, dKh over the heads of a group and over the tokens.
+extern "C" int cm_head_reduce(const void* dh, void* dgrp, float* dbias, long long T, int H, int G, int C, cudaStream_t s);
 extern "C" int cm_mimo_scan_bwd(const void* Qn, const void* Kn, const void* V, const void* Z, const void* dY,
                                 const float* ADT, const float* DT, const float* Trap, const float* Qb, const float* Kb,
                                 const float* Psi, const float* Zeta, const float* Phi, const float* angles,
                                 const float* Dskip, const void* states, const float* tot, float* gbuf, void* dend,
                                 void* dQh, void* dKh, void* dV, void* dZ, float* dAngles, float* dADT, float* dTs,
-                                float* dGam, float* dPsi, float* dZeta, float* dPhi, float* dD_, int B, int S, int H, int G,
+                                float* dGam, float* dPsi, float* dZeta, float* dPhi, float* dD_, float* dDT, float* dTrap, void* dQg,
+                                void* dKg, float* dQb, float* dKb, int B, int S, int H, int G,
                                 int N, long long ldV, long long ldZ, int* err, cudaStream_t stream) {
   if (B <= 0 || S <= 0) return 0;
   if (S % LT || N != 128 || H % G) return -10;
@@ -769,7 +798,7 @@ extern "C" int cm_mimo_scan_bwd(const void* Qn, const void* Kn, const void* V, c
   if (rc) return rc;
   BwdArgs a{(const __nv_bfloat16*)V, (const __nv_bfloat16*)Z, (const __nv_bfloat16*)dY, ADT, DT, Trap, Qb, Kb, Psi, Zeta,
             Phi, angles, Dskip, gbuf, (__nv_bfloat16*)dQh, (__nv_bfloat16*)dKh, (__nv_bfloat16*)dV, (__nv_bfloat16*)dZ,
-            dAngles, dADT, dTs, dGam, dPsi, dZeta, dPhi, dD_, B, S, H, G, C, ldV, ldZ, err, B * H * C};
+            dAngles, dADT, dTs, dGam, dPsi, dZeta, dPhi, dD_, dQg ? dQb : nullptr, dKb, B, S, H, G, C, ldV, ldZ, err, B * H * C};
   auto k0 = mimo_grad_state_kernel<128, 32>;
   auto k2 = mimo_chunk_grad_kernel<128, 32>;
   static PerDevice cfg;
@@ -783,6 +812,15 @@ extern "C" int cm_mimo_scan_bwd(const void* Qn, const void* Kn, const void* V, c
   dim3 g2(B * H, (128 * P + 1023) / 1024);
   mimo_state_scan_rev_kernel<<<g2, 256, 0, stream>>>(gbuf, tot, (__nv_bfloat16*)dend, C, 128 * P);
   k2<<<grid < sm_count() ? grid : sm_count(), THREADS2, chunk_grad_smem(), stream>>>(tmQ, tmK, tmS, tmE, a);
+  const long long n = (long long)B * H * S;
+  const long long blocks = (n + 255) / 256;
+  mimo_trapezoid_grad_kernel<<<(unsigned)(blocks < sm_count() * 8ll ? blocks : sm_count() * 8ll), 256, 0, stream>>>(dTs, dGam, DT, Trap, dDT,
+                                                                                                                  dTrap, n, S);
+  if (dQg) {
+    rc = cm_head_reduce(dQh, dQg, dQb, (long long)B * S, H, G, R * N, stream);
+    if (!rc) rc = cm_head_reduce(dKh, dKg, dKb, (long long)B * S, H, G, R * N, stream);
+    if (rc) return rc;
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

@@ -1,5 +1,5 @@
-"""Python side of the fused Mamba3 MIMO scan backward: launches the kernels and finishes the small
-reductions (heads -> groups, per-head biases, trapezoid coefficients -> DT / Trap)."""
+"""Python side of the fused Mamba3 MIMO scan backward: allocates and launches the kernels (a head count per group without a
+reduction kernel is reduced by the tensor library)."""
 from __future__ import annotations
 
 import torch
@@ -30,24 +30,26 @@ def mimo_bwd(saved, dy, states, tot):
     dADT = torch.empty(B, H, S, dtype=torch.float32, device=dev)
     dTs = torch.empty(B, H, S, dtype=torch.float32, device=dev)
     dGam = torch.empty(B, H, S, dtype=torch.float32, device=dev)
-    dPsi = torch.zeros(H, R, P, dtype=torch.float32, device=dev)
-    dZeta = torch.zeros(H, R, P, dtype=torch.float32, device=dev)
-    dPhi = torch.zeros(H, R, P, dtype=torch.float32, device=dev)
-    dD = torch.zeros(H, dtype=torch.float32, device=dev)
+    alloc = torch.empty if B * S else torch.zeros                                  # nothing is launched for an empty batch
+    e32 = lambda *shape: alloc(*shape, dtype=torch.float32, device=dev)
+    dPsi, dZeta, dPhi, dD = e32(H, R, P), e32(H, R, P), e32(H, R, P), e32(H)      # zeroed by the first kernel
+    dDT, dTrap = e32(B, H, S), e32(B, H, S)
+    grouped = hpg in (1, 2, 4, 8, 16)
+    if grouped:     # heads -> groups (Q/K are shared by the heads of a group) and per-head biases, one pass per tensor
+        dQg, dKg = (torch.empty(B, S, G, R, N, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        dQb, dKb = e32(H, R, N), e32(H, R, N)
     Vs, ldV = token_strided(V)
     Zs, ldZ = token_strided(Z)
     ins = [Qn, Kn, Vs, Zs, dyc, ADTf, DTf, Trapf, f32(Qb), f32(Kb), f32(Psi), f32(Zeta), f32(Phi),
            f32(angles), f32(D), states, tot]
-    outs = [gbuf, dend, dQh, dKh, dV, dZ, dAng, dADT, dTs, dGam, dPsi, dZeta, dPhi, dD]
-    _check(lib().cm_mimo_scan_bwd(*[t.data_ptr() for t in ins], *[t.data_ptr() for t in outs], B, S, H, G, N, ldV, ldZ,
+    outs = [gbuf, dend, dQh, dKh, dV, dZ, dAng, dADT, dTs, dGam, dPsi, dZeta, dPhi, dD, dDT, dTrap]
+    reduced = [t.data_ptr() for t in (dQg, dKg, dQb, dKb)] if grouped else [None] * 4
+    _check(lib().cm_mimo_scan_bwd(*[t.data_ptr() for t in ins], *[t.data_ptr() for t in outs], *reduced, B, S, H, G, N, ldV, ldZ,
                                   err_word(dev).data_ptr(), stream_ptr()), "cm_mimo_scan_bwd")
     F_.count_launch("mimo_scan_bwd", 3)
     del gbuf, dend
-    # heads -> groups (Q/K are shared by the heads of a group) and per-head biases, one pass per tensor
-    from .kernels4 import head_reduce
-    if hpg in (1, 2, 4, 8, 16):
-        dQg, dQb = head_reduce(dQh, G)
-        dKg, dKb = head_reduce(dKh, G)
+    if grouped:
+        F_.count_launch("head_reduce", 2)
         dQ, dK = dQg.permute(0, 1, 3, 2, 4), dKg.permute(0, 1, 3, 2, 4)
     else:
         dQ = dQh.view(B, S, G, hpg, R, N).sum(3, dtype=torch.float32).permute(0, 1, 3, 2, 4)
@@ -55,13 +57,6 @@ def mimo_bwd(saved, dy, states, tot):
         dQb = dQh.sum((0, 1), dtype=torch.float32)
         dKb = dKh.sum((0, 1), dtype=torch.float32)
     del dQh, dKh
-    # trapezoid coefficients: gamma_t = DT_t sig(Trap_t), ts_t = gamma_t + DT_{t+1} sig(-Trap_{t+1})
-    sg = torch.sigmoid(Trapf)
-    dgt = dGam + dTs
-    prev = torch.zeros_like(dTs)
-    prev[..., 1:] = dTs[..., :-1]
-    dDT = dgt * sg + prev * (1.0 - sg)
-    dTrap = (dgt - prev) * DTf * sg * (1.0 - sg)
     return (dQ.to(Q.dtype), dK.to(K.dtype), dV.to(V.dtype), dADT.to(ADT.dtype), dDT.to(DT.dtype), dTrap.to(Trap.dtype),
             dQb.to(Qb.dtype), dKb.to(Kb.dtype), dPsi.to(Psi.dtype), dZeta.to(Zeta.dtype), dPhi.to(Phi.dtype),
             dAng.to(angles.dtype), dD.to(D.dtype), dZ.to(Z.dtype))
