@@ -5,7 +5,7 @@
 //
 // forward   one CTA per (pair of 128-query tiles, head, batch).  A TMA warp keeps up to three (K, V) tiles in shared memory, an
 //           MMA warp issues S_t = Q_t K^T and O_t += P_t V for the two query tiles t in turn, and one warpgroup per query
-//           tile (thread <-> query row <-> TMEM lane) does the softmax: S is read twice (maximum, exponentials), P goes back to
+//           tile (thread <-> query row <-> TMEM lane) does the softmax: half of S is read twice (maximum, exponentials), P goes back to
 //           TMEM as the bf16 A operand of P V, and O stays in TMEM.  O is rescaled only when a row maximum has grown by more
 //           than 2^8 since the last rescale (the softmax is the same for any reference value; l and O use the same one).
 //           What bounds it: the exponentials, 128 x 128 of them per tile at 16 a cycle = 1024 cycles against 768 of tensor
@@ -21,8 +21,9 @@
 //           staging a tile are about 3,700 cycles at 128 bytes a cycle, against 2,048 of tensor work.
 // All operand tiles are 128-byte-swizzled [128 x 64] bf16 slabs written by TMA (2-D maps over [B*S, H*dim]); the same
 // slab is read K-major or MN-major by choosing the descriptor.  Every wait is bounded and reports through the error word.
-// Measured at batch 2, seq 4096, 32 heads: forward 276 us (633 with one 128-thread CTA per query tile, K and V loaded in line and
-// two passes of exp2f with range handling), backward 755 us (1660 with 128 threads walking the phases one after the other).
+// Measured at batch 2, seq 4096, 32 heads: forward 262 us (633 with one 128-thread CTA per query tile, K and V loaded in line and
+// two passes of exp2f with range handling), backward 697 us (1660 with 128 threads walking the phases one after the other; 587
+// when the dQ reductions are left out, so they are a sixth of it).
 // The reference takes this operator from cuDNN / FlashAttention (`--attention-backend flash`,
 // scripts/remote_smoke_h200_dsa_9_4_m.sh:727-728; MLA adapter at cppmega/megatron/mla_shared.py:39-97).
 #include "common.cuh"
@@ -227,10 +228,11 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_kernel(const __grid_c
       bool ok = warp_wait(&sh->s_full[t], j & 1, abort_flag, a.err, ERR_WAIT_TMEM_FULL);
       if (!ok) return false;
       tc_fence_after();
-      float m_new = -INFINITY;              // first pass over the row: its maximum
+      // first pass over the row: its maximum.  The first half of the row is read last and kept for the second pass.
+      float m_new = -INFINITY;
+      uint32_t s0[32], s1[32], s2[32];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t s0[32], s1[32];
+      for (int c = 1; c >= 0; --c) {
         tmem_ld_32x32(tS + c * 64, s0);
         tmem_ld_32x32(tS + c * 64 + 32, s1);
         tmem_ld_wait();
@@ -266,33 +268,34 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_kernel(const __grid_c
         }
       }
       float sum[4] = {0.f, 0.f, 0.f, 0.f};  // second pass: P in bf16, row sum in fp32
+      uint32_t p[32];
+      auto quarter = [&](const uint32_t (&sc)[32], int col0, int at) {
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        uint32_t p[32];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t s0[32];
-          tmem_ld_32x32(tS + hf * 64 + c * 32, s0);
-          tmem_ld_wait();
-#pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            float x = ex2(fmaf(__uint_as_float(s0[2 * e]), a.scale_log2, -m_ref));
-            float y = ex2(fmaf(__uint_as_float(s0[2 * e + 1]), a.scale_log2, -m_ref));
-            if (DIAG) {
-              x = hf * 64 + c * 32 + 2 * e <= r ? x : 0.f;
-              y = hf * 64 + c * 32 + 2 * e + 1 <= r ? y : 0.f;
-            }
-            sum[(2 * e) & 3] += x;
-            sum[(2 * e + 1) & 3] += y;
-            p[c * 16 + e] = pack_bf16(x, y);
+        for (int e = 0; e < 16; ++e) {
+          float x = ex2(fmaf(__uint_as_float(sc[2 * e]), a.scale_log2, -m_ref));
+          float y = ex2(fmaf(__uint_as_float(sc[2 * e + 1]), a.scale_log2, -m_ref));
+          if (DIAG) {
+            x = col0 + 2 * e <= r ? x : 0.f;
+            y = col0 + 2 * e + 1 <= r ? y : 0.f;
           }
+          sum[(2 * e) & 3] += x;
+          sum[(2 * e + 1) & 3] += y;
+          p[at + e] = pack_bf16(x, y);
         }
-        tmem_st_32x32(tP + hf * 32, p);
-      }
-      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      };
+      quarter(s0, 0, 0);
+      quarter(s1, 32, 16);
+      tmem_st_32x32(tP, p);
+      tmem_ld_32x32(tS + 64, s2);
+      tmem_ld_32x32(tS + 96, s1);
+      tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->s_free[t]);
+      quarter(s2, 64, 0);
+      quarter(s1, 96, 16);
+      tmem_st_32x32(tP + 32, p);
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -366,8 +369,20 @@ struct BwdArgs {
   __nv_bfloat16* dv;    // [B, S, H, DV]
   int S, H, n_kt;
   float scale, scale_log2;
+  int heads_per_group;
   int* err;
 };
+
+// CTA -> ((batch, head), key tile in descending order of work).  Groups of heads that fill the SMs about once run one after the
+// other, so that the operands and the dQ rows in use stay in L2: with all heads at once 10.7 GB went through DRAM at batch 4,
+// seq 4096, of which 0.9 GB are needed (755 -> 700 us at batch 2).  The forward, whose operands are read only, keeps the order
+// over all heads: its longest CTAs then start first over the whole grid (276 us against 314 in groups).
+__device__ __forceinline__ void decode_cta(int x, int tiles, int heads, int per_group, int& bh, int& tile) {
+  const int grp = x / (per_group * tiles), in = x - grp * per_group * tiles;
+  const int n = min(per_group, heads - grp * per_group);
+  tile = in / n;
+  bh = grp * per_group + in - tile * n;
+}
 
 constexpr int BWD_THREADS = 448;          // warps 0-7: P and dS (warp >> 2 = half of the key columns); 8-11: dQ; 12: MMA; 13: TMA
 
@@ -411,9 +426,8 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   BwdShared* sh = reinterpret_cast<BwdShared*>(sdQ + SLAB);
   if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
 
-  // key tile 0 has the longest loop: it goes first
-  const int bh = blockIdx.x % (gridDim.x / a.n_kt);
-  const int kt = blockIdx.x / (gridDim.x / a.n_kt);
+  int bh, kt;                               // key tile 0 has the longest loop
+  decode_cta(blockIdx.x, a.n_kt, gridDim.x / a.n_kt, a.heads_per_group, bh, kt);
   const int h = bh % a.H, b = bh / a.H;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int k0 = kt * BK;
@@ -700,7 +714,8 @@ extern "C" int cm_attn_bwd(const void* q, const void* k, const void* v, const vo
   attn_delta_kernel<<<(unsigned)((nrows + 31) / 32), 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta,
                                                                       nrows, S, H);
   const int n_kt = S / BK;
-  BwdArgs a{lse2, delta, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, S, H, n_kt, scale, scale * 1.4426950408889634f, err};
+  BwdArgs a{lse2, delta, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv, S, H, n_kt, scale, scale * 1.4426950408889634f,
+            (sm_count() + n_kt - 1) / n_kt, err};
   attn_bwd_kernel<<<(unsigned)(n_kt * B * H), BWD_THREADS, bwd_smem(), stream>>>(tmQ, tmK, tmV, tmdO, tmdQ, a);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
