@@ -141,6 +141,9 @@ __global__ void __launch_bounds__(THREADS2) mimo_grad_state_kernel(const __grid_
   const float4 ang4 = load_angles4<NROT>(a.angles, b, t0, h, a.S, a.H);
   const HalfRowRaw yraw = load_half_raw(a.dY, b, t0, h, a.S, (long long)a.H * P);
   const HalfRowRaw zraw = load_half_raw(a.Z, b, t0, h, a.S, a.ldZ);
+  const float* qbh = a.Qb + (size_t)h * R * N + 2 * threadIdx.x;
+  const float qb0 = qbh[0], qb1 = qbh[1];
+  const float zeta1 = a.Zeta[(size_t)h * R * P + threadIdx.x], phi1 = a.Phi[(size_t)h * R * P + threadIdx.x];
   if (threadIdx.x == 0) {
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
@@ -157,7 +160,13 @@ __global__ void __launch_bounds__(THREADS2) mimo_grad_state_kernel(const __grid_
 #pragma unroll
     for (int s = 0; s < N / 64; ++s) tma_load_5d_b(sQ + s * SLAB, &tmQ, &bars[0], s * 64, 0, g, t0, b);
   }
-  load_head_consts<N>(hb, hv, a.Qb, a.Qb, a.Phi, a.Zeta, a.Phi, h);
+  {
+    const int bias_at = (2 * threadIdx.x / N) * HeadBias<N>::LD + 2 * threadIdx.x % N;
+    hb->qb[bias_at] = qb0;
+    hb->qb[bias_at + 1] = qb1;
+    hv->zeta[vec_idx(threadIdx.x)] = zeta1;
+    hv->phi[vec_idx(threadIdx.x)] = phi1;
+  }
   finish_chunk_scalars(sc, sl, t0, a.S);
   fill_sincos4<NROT>(cos_tab, sin_tab, ang4);
   __syncthreads();
@@ -185,16 +194,8 @@ __global__ void __launch_bounds__(THREADS2) mimo_grad_state_kernel(const __grid_
   }
   ok = mbar_wait(&bars[1], 0, abort_flag, a.err, ERR_WAIT_TMEM_FULL);
   tc_fence_after();
-  if (ok) {
-    float* dst = a.gbuf + ((((size_t)b * a.H + h) * a.C + c) * N + i) * P + wg * 32;
-    uint32_t rr[32];
-    tmem_ld_32x32(tmem + (uint32_t((warp & 3) * 32) << 16) + wg * 32, rr);
-    tmem_ld_wait();
-#pragma unroll
-    for (int v = 0; v < 8; ++v)
-      reinterpret_cast<float4*>(dst)[v] = make_float4(__uint_as_float(rr[4 * v]), __uint_as_float(rr[4 * v + 1]),
-                                                      __uint_as_float(rr[4 * v + 2]), __uint_as_float(rr[4 * v + 3]));
-  }
+  static_assert(N == ROWS, "one TMEM lane per state row");
+  store_state_tile(a.gbuf + (((size_t)b * a.H + h) * a.C + c) * N * P, sQ, tmem, ok);
   tc_fence_before();
   __syncthreads();
   if (warp == 0) { tc_fence_after(); tmem_dealloc(tmem, 64); }

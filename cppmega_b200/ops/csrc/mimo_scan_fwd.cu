@@ -100,11 +100,14 @@ __global__ void __launch_bounds__(THREADS2) mimo_local_state_kernel(const __grid
   int b, g, c, h;
   decode_block(a, b, g, c, h);
   const int t0 = c * LT;
-  const int warp = threadIdx.x >> 5, i = threadIdx.x & 127, wg = threadIdx.x >> 7;
+  const int warp = threadIdx.x >> 5, i = threadIdx.x & 127;
   // every global load of the prologue is issued here, ahead of the set-up, and consumed further down
   const ScalarLoads sl = load_chunk_scalars(a.ADT, a.DT, a.Trap, ((size_t)b * a.H + h) * a.S + t0, t0, a.S);
   const float4 ang4 = load_angles4<NROT>(a.angles, b, t0, h, a.S, a.H);
   const HalfRowRaw vraw = load_half_raw(a.V, b, t0, h, a.S, a.ldV);
+  static_assert(R * N == 2 * THREADS2 && R * P == THREADS2, "two bias elements and one psi element per thread");
+  const float* kbh = a.Kb + (size_t)h * R * N + 2 * threadIdx.x;
+  const float kb0 = kbh[0], kb1 = kbh[1], psi1 = a.Psi[(size_t)h * R * P + threadIdx.x];
   if (threadIdx.x == 0) {
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
@@ -121,7 +124,12 @@ __global__ void __launch_bounds__(THREADS2) mimo_local_state_kernel(const __grid
 #pragma unroll
     for (int s = 0; s < N / 64; ++s) tma_load_5d(sK + s * SLAB, &tmK, &bars[0], s * 64, 0, g, t0, b);
   }
-  load_head_consts<N>(hb, hv, nullptr, a.Kb, a.Psi, nullptr, nullptr, h);
+  {
+    const int bias_at = (2 * threadIdx.x / N) * HeadBias<N>::LD + 2 * threadIdx.x % N;
+    hb->kb[bias_at] = kb0;
+    hb->kb[bias_at + 1] = kb1;
+    hv->psi[vec_idx(threadIdx.x)] = psi1;
+  }
   finish_chunk_scalars(sc, sl, t0, a.S);
   fill_sincos4<NROT>(cos_tab, sin_tab, ang4);
   __syncthreads();
@@ -145,16 +153,8 @@ __global__ void __launch_bounds__(THREADS2) mimo_local_state_kernel(const __grid
   }
   ok = mbar_wait(&bars[1], 0, abort_flag, a.err, ERR_WAIT_TMEM_FULL);
   tc_fence_after();
-  if (ok) {
-    float* dst = a.local + ((((size_t)b * a.H + h) * a.C + c) * N + i) * P + wg * 32;
-    uint32_t r[32];
-    tmem_ld_32x32(tmem + (uint32_t((warp & 3) * 32) << 16) + wg * 32, r);
-    tmem_ld_wait();
-#pragma unroll
-    for (int v = 0; v < 8; ++v)
-      reinterpret_cast<float4*>(dst)[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]),
-                                                      __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-  }
+  static_assert(N == ROWS, "one TMEM lane per state row");
+  store_state_tile(a.local + (((size_t)b * a.H + h) * a.C + c) * N * P, sK, tmem, ok);
   if (threadIdx.x == 0) a.tot[((size_t)b * a.H + h) * a.C + c] = sc->tot;
   tc_fence_before();
   __syncthreads();
