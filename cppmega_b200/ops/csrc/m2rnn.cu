@@ -8,10 +8,13 @@
 // keep fp32 operands: W is bf16 as given, and the fp32 factor is the sum of three bf16 parts (8 + 8 + 8 mantissa bits), each
 // multiplied exactly and added in fp32.
 //
-// What bounds it: the chain of dependent steps, not arithmetic or memory (one warp per scheduler; 4096 steps).  With four
+// What bounds it: the instructions of a step - one warp per scheduler, each instruction 2.3 cycles at the dependences of a chain -
+// not arithmetic or memory.  So every sum that can be one is a matrix product: the gradients of k and q against an operand
+// with v and dy in two of its columns, the gradient of v against one with k in a row.  With four
 // threads per row, 12 shuffles and 64 dependent multiply-adds a step and the state history fetched one step ahead, the
-// backward took 1.23 us and the forward 0.29 us a step at batch 2, 51 heads; now 0.49 and 0.26 (the history is requested four
-// steps ahead, and a warp issues 378 instructions a backward step).
+// backward took 1.23 us and the forward 0.29 us a step at batch 2, 51 heads; now 0.44 and 0.26 (1,793 us and 1,078 us in all).
+// The history is requested four steps ahead.  Two warps per 16 rows, the second forming the gradients a block of steps behind,
+// were slower (0.61 us a step: 589 instructions between them instead of 378 then in one warp).
 // Only dh_{t-1} = f_t dh_t + da_t W^T is on the backward's chain; the replay of tanh(a_t) and all other gradients hang off it.
 //
 // Inputs are staged through shared memory in blocks of 16 steps (the next block is loaded into registers while the current
@@ -49,26 +52,32 @@ __device__ __forceinline__ void split3(const float (&c)[8], Split3& s) {
     s.lo[p] = pack_bf16(x, y);
   }
 }
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+// d = a b + c.  Sums start from a constant or from a term of the step, so that no accumulator is cleared or added separately.
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2], const float (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
-// out[0..3] | out[4..7] = x M for the 16 x 16 bf16 matrix M held as B fragments
-__device__ __forceinline__ void times16(float (&out)[8], const Split3& x, const uint32_t (&m)[2][2]) {
+__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  const float z[4] = {0.f, 0.f, 0.f, 0.f};
+  mma16816(d, a, b, z);
+}
+// out = (lo + mid) M on top of `init`, plus hi M: the large part is added last, in fp32 rounding
+__device__ __forceinline__ void times16(float (&out)[8], const Split3& x, const uint32_t (&m)[2][2], const float (&init)[8]) {
 #pragma unroll
   for (int n = 0; n < 2; ++n) {
-    float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
-    mma16816(a, x.lo, m[n]);
+    float a[4], b[4];
+    const float c[4] = {init[n * 4], init[n * 4 + 1], init[n * 4 + 2], init[n * 4 + 3]};
+    mma16816(a, x.lo, m[n], c);
     mma16816(b, x.hi, m[n]);
-    mma16816(a, x.mid, m[n]);
+    mma16816(a, x.mid, m[n], a);
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[n * 4 + i] = a[i] + b[i];
   }
 }
 __device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
   uint32_t y;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
   return y;
 }
 // Sum of x[0..3] over the 8 lanes with equal (lane & 3); lane returns the sum of element 2 * bit4 + bit3 (bit2 is redundant).
@@ -100,6 +109,9 @@ __device__ __forceinline__ void spread8(float* dst, uint4 v) {
 template <int KD, bool BWD>
 struct Stage {
   float q[TB][KD], k[TB][KD], v[TB][VD], g[BWD ? TB : 1][VD], f[TB];
+  // the backward also wants k, v and dy as they are, as MMA operands: pairs of bf16
+  __align__(16) uint32_t kb[BWD ? TB : 1][KD / 2];
+  __align__(16) uint32_t vg[BWD ? TB : 1][2][VD / 2];
 };
 
 template <int KD, bool BWD>
@@ -129,9 +141,14 @@ struct Loader {
     const int t = tid / (KD / 8), c = (tid % (KD / 8)) * 8;
     spread8(&s.q[t][c], rq);
     spread8(&s.k[t][c], rk);
+    if (BWD) *reinterpret_cast<uint4*>(&s.kb[BWD ? t : 0][c / 2]) = rk;
     if (tid < 2 * TB) {
       spread8(&s.v[tid >> 1][(tid & 1) * 8], rv);
-      if (BWD) spread8(&s.g[tid >> 1][(tid & 1) * 8], rg);
+      if (BWD) {
+        spread8(&s.g[BWD ? tid >> 1 : 0][(tid & 1) * 8], rg);
+        *reinterpret_cast<uint4*>(&s.vg[BWD ? tid >> 1 : 0][0][(tid & 1) * 4]) = rv;
+        *reinterpret_cast<uint4*>(&s.vg[BWD ? tid >> 1 : 0][1][(tid & 1) * 4]) = rg;
+      }
       if (tid < TB) s.f[tid] = rf;
     }
   }
@@ -204,15 +221,13 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_fwd_kernel(
       const float vv[4] = {va.x, va.y, vb.x, vb.y};
       Split3 s;
       split3(hs, s);
-      float a[8];
-      times16(a, s, w);
-      float yp[4];
+      float a[8], kv[8], yp[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int c = (i >> 2) * 2 + (i & 1);      // column slot of element i; elements 2, 3, 6, 7 are row r0 + 8
-        const float x = fmaf((i & 2) ? k1 : k0, vv[c], a[i]);
-        hs[i] = fmaf(ft, hs[i], (1.f - ft) * fast_tanh(x));
-      }
+      for (int i = 0; i < 8; ++i) kv[i] = ((i & 2) ? k1 : k0) * vv[(i >> 2) * 2 + (i & 1)];    // elements 2, 3, 6, 7 are row r0 + 8
+      times16(a, s, w, kv);
+      const float omf = 1.f - ft;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) hs[i] = fmaf(ft, hs[i], omf * fast_tanh(a[i]));
       if (hist) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -275,16 +290,22 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
   for (int i = tid; i < VD * VD; i += NT) (&sh.dw[0][0])[i] = 0.f;
   const float* hbase = hist + ((size_t)blockIdx.x * S * KD + r0) * VD + 2 * t4;
   auto load_state = [&](float (&x)[8], int t) {   // h_t, zero before the first step and (never used) past the last
+    const float* hp = hbase + (long long)t * (KD * VD);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float2 p = make_float2(0.f, 0.f);
-      if (t >= 0 && t < S) p = *reinterpret_cast<const float2*>(hbase + (size_t)t * KD * VD + ((i & 1) ? 8 * VD : 0) + (i >> 1) * 8);
+      if (t >= 0 && t < S) p = *reinterpret_cast<const float2*>(hp + ((i & 1) ? 8 * VD : 0) + (i >> 1) * 8);
       x[2 * i] = p.x; x[2 * i + 1] = p.y;
     }
   };
   const int nblocks = (S + TB - 1) / TB;
-  float hcur[8], ring[AHEAD][8], dh[8], dw_sum[2][4];
-  load_state(hcur, S - 1);
+  float ring[AHEAD][8], dh[8], dw_sum[2][4];
+  Split3 hcur;                                    // h_t of the step at hand
+  {
+    float h_end[8];
+    load_state(h_end, S - 1);
+    split3(h_end, hcur);
+  }
 #pragma unroll
   for (int i = 0; i < AHEAD; ++i) load_state(ring[AHEAD - 1 - i], nblocks * TB - 2 - i);     // slot of step s: s % AHEAD, holds h_{s-1}
 #pragma unroll
@@ -295,7 +316,7 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
     for (int i = 0; i < 4; ++i) dw_sum[n][i] = 0.f;
   in.fetch((nblocks - 1) * TB, tid);
   in.commit(sh.stage[(nblocks - 1) & 1], tid);
-  const int col = reduced_col(lane);
+  const uint32_t row0_mask = g == 0 ? 0xffffffffu : 0u, col01_mask = g < 2 ? 0xffffffffu : 0u;
   auto write_out = [&](int blk) {                 // the gradients of block `blk` from its shared-memory parts
     const int t0 = blk * TB, nt = min(TB, S - t0), p = blk & 1;
     for (int e = tid; e < nt * KD; e += NT) {
@@ -351,64 +372,71 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
         // replay of tanh(a_t); off the chain
         Split3 sp;
         split3(hprev, sp);
-        float a[8];
-        times16(a, sp, w);
-        float da[8], dfp = 0.f, red[4] = {0.f, 0.f, 0.f, 0.f};      // red: dq of rows r0, r0 + 8, dk of the same
+        float a[8], kv[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) kv[i] = ((i & 2) ? k1 : k0) * vv[(i >> 2) * 2 + (i & 1)];
+        times16(a, sp, w, kv);
+        float da[8], dfp = 0.f;
+        const float omf = 1.f - ft;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int c = (i >> 2) * 2 + (i & 1), up = (i >> 1) & 1;
-          const float hn = fast_tanh(fmaf(up ? k1 : k0, vv[c], a[i]));
-          dh[i] = fmaf(up ? q1 : q0, gg[c], dh[i]);
-          red[up] = fmaf(hcur[i], gg[c], red[up]);
+          const float hn = fast_tanh(a[i]);
+          dh[i] = fmaf((i & 2) ? q1 : q0, gg[(i >> 2) * 2 + (i & 1)], dh[i]);
           dfp = fmaf(dh[i], hprev[i] - hn, dfp);
-          da[i] = dh[i] * ((1.f - ft) * (1.f - hn * hn));
-          red[2 + up] = fmaf(da[i], vv[c], red[2 + up]);
+          da[i] = dh[i] * fmaf(-omf, hn * hn, omf);
         }
         Split3 sd;
         split3(da, sd);
         float back[8];
-        times16(back, sd, wt);
+        const float none[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        times16(back, sd, wt, none);
 #pragma unroll
         for (int i = 0; i < 8; ++i) dh[i] = fmaf(ft, dh[i], back[i]);
-        // dW[u][v] += sum_rows h_{t-1}[row][u] da[row][v]: both factors transposed within the warp, six products of parts
+        // dk[row] = sum_v da[row][v] v[v], dq[row] = sum_v h_t[row][v] dy[v]: one operand with v in column 0 and dy in column 1
         {
-          uint32_t ht[3][4], dt[3][4];
+          const uint32_t vg[2] = {st.vg[t][g & 1][t4] & col01_mask, st.vg[t][g & 1][4 + t4] & col01_mask};
+          float rk[4], rq[4];
+          mma16816(rk, sd.lo, vg);
+          mma16816(rq, hcur.lo, vg);
+          mma16816(rk, sd.mid, vg, rk);
+          mma16816(rq, hcur.mid, vg, rq);
+          mma16816(rk, sd.hi, vg, rk);
+          mma16816(rq, hcur.hi, vg, rq);
+          if (t4 == 0) {
+            sh.dk[p][t][r0] = rk[0];
+            sh.dk[p][t][r0 + 8] = rk[2];
+            sh.dq[p][t][r0] = rq[1];
+            sh.dq[p][t][r0 + 8] = rq[3];
+          }
+        }
+        // dW[u][v] += sum_rows h_{t-1}[row][u] da[row][v] and dv[v] = sum_rows k[row] da[row][v]: da as the right factor, h as the
+        // left one, both transposed within the warp.  Two parts of each (16 mantissa bits; k is exact): the sums are rounded to bf16.
+        {
+          uint32_t hh[4], hm[4], dd[4], dm[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int j = (i & 1) * 2 + (i >> 1);  // block (row half, column half) -> (column half, row half)
-            ht[0][j] = transpose8x8(sp.hi[i]); ht[1][j] = transpose8x8(sp.mid[i]); ht[2][j] = transpose8x8(sp.lo[i]);
-            dt[0][i] = transpose8x8(sd.hi[i]); dt[1][i] = transpose8x8(sd.mid[i]); dt[2][i] = transpose8x8(sd.lo[i]);
+            hh[j] = transpose8x8(sp.hi[i]); hm[j] = transpose8x8(sp.mid[i]);
+            dd[i] = transpose8x8(sd.hi[i]); dm[i] = transpose8x8(sd.mid[i]);
           }
+          const uint32_t kr[4] = {st.kb[t][warp * 8 + t4] & row0_mask, 0u, st.kb[t][warp * 8 + 4 + t4] & row0_mask, 0u};
+          float dvp[2][4];
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
-#pragma unroll
-            for (int x = 2; x >= 0; --x)
-#pragma unroll
-              for (int z = 2 - x; z >= 0; --z) {
-                const uint32_t bb[2] = {dt[z][n * 2], dt[z][n * 2 + 1]};
-                mma16816(dw_blk[n], ht[x], bb);
-              }
+            const uint32_t bh[2] = {dd[n * 2], dd[n * 2 + 1]}, bm[2] = {dm[n * 2], dm[n * 2 + 1]};
+            mma16816(dvp[n], kr, bm);
+            mma16816(dw_blk[n], hm, bh, dw_blk[n]);
+            mma16816(dvp[n], kr, bh, dvp[n]);
+            mma16816(dw_blk[n], hh, bm, dw_blk[n]);
+            mma16816(dw_blk[n], hh, bh, dw_blk[n]);
+          }
+          if (g == 0) {
+            *reinterpret_cast<float2*>(&sh.dv[p][t][warp][2 * t4]) = make_float2(dvp[0][0], dvp[0][1]);
+            *reinterpret_cast<float2*>(&sh.dv[p][t][warp][8 + 2 * t4]) = make_float2(dvp[1][0], dvp[1][1]);
           }
         }
-        // dq, dk: sum over the four lanes of a row; each lane ends with one of the four
-        {
-          const bool o1 = lane & 1, o2 = lane & 2;
-          const float x0 = (o1 ? red[2] : red[0]) + __shfl_xor_sync(0xffffffffu, o1 ? red[0] : red[2], 1);
-          const float x1 = (o1 ? red[3] : red[1]) + __shfl_xor_sync(0xffffffffu, o1 ? red[1] : red[3], 1);
-          const float r = (o2 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, o2 ? x0 : x1, 2);
-          (o1 ? sh.dk : sh.dq)[p][t][r0 + (o2 ? 8 : 0)] = r;
-        }
-        float dvp[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int i = (c >> 1) * 4 + (c & 1);
-          dvp[c] = fmaf(da[i + 2], k1, da[i] * k0);
-        }
-        const float r = reduce_rows4(dvp, lane);
-        if ((lane & 4) == 0) sh.dv[p][t][warp][col] = r;
         sh.df[p][t][tid] = dfp;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) hcur[i] = hprev[i];
+        hcur = sp;
       }
     }
 #pragma unroll
