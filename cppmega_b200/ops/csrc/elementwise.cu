@@ -327,8 +327,8 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_small(const __nv_bfloat16* __
 // counts is the bytes in flight and the latency of a row's block-wide sum.  Every thread copies its own vectors of the next NS
 // groups of rows into shared memory with asynchronous copies and reads back only what it copied, so the copies need no
 // barrier, and the one barrier of a group (its sums alternate between two buffers) leaves them running; the U sums of a
-// group share its latency.  16,384 x 4096: 100 us (61 at the copy rate), 166 with one row per CTA
-// pass, two barriers and one row prefetched into registers.
+// group share its latency.  16,384 x 4096: 73 us (61 at the copy rate); 100 with dw added one float at a time, 166 with one row
+// per CTA pass, two barriers and one row prefetched into registers as well.
 template <int TPB, int VPT, int U, int NS>
 __global__ void __launch_bounds__(TPB) rmsnorm_bwd_ring(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                         const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd_in,
@@ -468,14 +468,21 @@ __global__ void __launch_bounds__(TPB) rmsnorm_bwd_ring(const __nv_bfloat16* __r
     }
   }
   if (dw) {
+    // All CTAs add to the same H floats at the same time: through shared memory a warp instruction adds 512 consecutive bytes
+    // (straight from the registers it touches one float in each of 32 sectors).
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                            // the ring is free
+    float4* sum = reinterpret_cast<float4*>(ring);
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int idx = tid + i * TPB;
       if (idx < nvec) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) atomicAdd(dw + idx * 8 + j, dwacc[i][j]);
+        sum[2 * idx] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
+        sum[2 * idx + 1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
       }
     }
+    __syncthreads();
+    for (int c = tid; c < 2 * nvec; c += TPB) atomicAdd(reinterpret_cast<float4*>(dw) + c, sum[c]);
   }
 }
 
