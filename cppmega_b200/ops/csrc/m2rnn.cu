@@ -12,7 +12,7 @@
 // not arithmetic or memory.  So every sum that can be one is a matrix product: the gradients of k and q against an operand
 // with v and dy in two of its columns, the gradient of v against one with k in a row.  With four
 // threads per row, 12 shuffles and 64 dependent multiply-adds a step and the state history fetched one step ahead, the
-// backward took 1.23 us and the forward 0.29 us a step at batch 2, 51 heads; now 0.44 and 0.26 (1,793 us and 1,078 us in all).
+// backward took 1.23 us and the forward 0.29 us a step at batch 2, 51 heads; now 0.44 and 0.26 (1,788 us and 1,082 us in all).
 // The history is requested four steps ahead.  Two warps per 16 rows, the second forming the gradients a block of steps behind,
 // were slower (0.61 us a step: 589 instructions between them instead of 378 then in one warp).
 // Only dh_{t-1} = f_t dh_t + da_t W^T is on the backward's chain; the replay of tanh(a_t) and all other gradients hang off it.
@@ -71,6 +71,24 @@ __device__ __forceinline__ void times16(float (&out)[8], const Split3& x, const 
     mma16816(a, x.lo, m[n], c);
     mma16816(b, x.hi, m[n]);
     mma16816(a, x.mid, m[n], a);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out[n * 4 + i] = a[i] + b[i];
+  }
+}
+// The forward's chain: the same with the products kept in this order (free to move, the compiler delays the first by the
+// instructions of the step's other work: 1,155 us against 1,082 at batch 2, 51 heads) and nothing to start from
+__device__ __forceinline__ void times16_in_order(float (&out)[8], const Split3& x, const uint32_t (&m)[2][2]) {
+  auto mma = [](float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+  };
+#pragma unroll
+  for (int n = 0; n < 2; ++n) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f}, b[4] = {0.f, 0.f, 0.f, 0.f};
+    mma(a, x.lo, m[n]);
+    mma(b, x.hi, m[n]);
+    mma(a, x.mid, m[n]);
 #pragma unroll
     for (int i = 0; i < 4; ++i) out[n * 4 + i] = a[i] + b[i];
   }
@@ -221,13 +239,12 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_fwd_kernel(
       const float vv[4] = {va.x, va.y, vb.x, vb.y};
       Split3 s;
       split3(hs, s);
-      float a[8], kv[8], yp[4];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) kv[i] = ((i & 2) ? k1 : k0) * vv[(i >> 2) * 2 + (i & 1)];    // elements 2, 3, 6, 7 are row r0 + 8
-      times16(a, s, w, kv);
+      float a[8], yp[4];
+      times16_in_order(a, s, w);
       const float omf = 1.f - ft;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) hs[i] = fmaf(ft, hs[i], omf * fast_tanh(a[i]));
+      for (int i = 0; i < 8; ++i)                  // elements 2, 3, 6, 7 are row r0 + 8
+        hs[i] = fmaf(ft, hs[i], omf * fast_tanh(fmaf((i & 2) ? k1 : k0, vv[(i >> 2) * 2 + (i & 1)], a[i])));
       if (hist) {
 #pragma unroll
         for (int i = 0; i < 4; ++i)
