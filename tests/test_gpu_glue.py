@@ -424,6 +424,31 @@ def test_moe_transport_skips_and_reports_rows_beyond_capacity():
     assert (d.view(T, k)[~keep] == 0).all()
 
 
+@pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("H", [8, 264, 520, 1024])
+def test_moe_pulls_over_rows_per_token_and_widths(k, H):
+    """Both pulls for row counts on either side of each kernel's limit and widths that leave a partial vector group."""
+    from cppmega_b200.parallel import fused_moe as fm
+    torch.manual_seed(k)
+    T, E = 37, 16
+    ids = torch.stack([torch.randperm(E, device="cuda")[:k] for _ in range(T)])
+    cap = 2 * E * fm.TILE
+    plan = fm.MoEPlan(ids, E, 1, 0, None, cap, None)
+    heap = fm._LocalHeap()
+    rows = torch.randn(cap, H, device="cuda").bfloat16()
+    w = torch.rand(T * k, device="cuda")
+    dy = torch.randn(T, H, device="cuda").bfloat16()
+    picked = rows.double()[plan.dest_row].view(T, k, H)
+    for weights in (w, None):
+        terms = picked * (w.double().view(T, k, 1) if weights is not None else 1.0)
+        y = fm._pull_combine(heap, rows, plan, weights, H, torch.bfloat16).double()
+        # k fp32 additions, then one rounding to bf16
+        assert ((y - terms.sum(1)).abs() <= 2.0 ** -8 * terms.sum(1).abs() + k * 2.0 ** -22 * terms.abs().sum(1)).all()
+    d = fm._pull_rowdot(heap, rows, plan, dy).double().view(T, k)
+    terms = picked * dy.double()[:, None]
+    assert ((d - terms.sum(2)).abs() <= (H // 32 + 8) * 2.0 ** -23 * terms.abs().sum(2)).all()
+
+
 def _tensorwise_q(t):
     """fp32 restatement of the tensorwise FP8 recipe: one power-of-two scale from the tensor's amax, E4M3 rounding."""
     from cppmega_b200.ops import reference as ref
