@@ -159,19 +159,22 @@ class LinearCEWeightedFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g_total, _g_per_tok):
-        from . import lib, stream_ptr, _check
         dh, dw = ctx.saved_tensors
-        if torch.is_grad_enabled():                    # create_graph: keep the product with the upstream factor differentiable
-            return dh * g_total.to(dh.dtype), (dw * g_total).to(ctx.w_dtype), None, None, None
-        g = g_total.float().reshape(1)
-        outs = []
-        for t in (dh, dw):                             # scaled and rounded to bf16 in one pass
-            o = torch.empty(t.shape, dtype=torch.bfloat16, device=t.device)
-            _check(lib().cm_scale_to_bf16(t.data_ptr(), int(t.dtype == torch.float32), o.data_ptr(), g.data_ptr(), t.numel(),
-                                          stream_ptr()), "cm_scale_to_bf16")
-            F_.count_launch("scale_to_bf16")
-            outs.append(o)
-        return outs[0], outs[1], None, None, None
+        return _scale_head_grad(dh, g_total, dh.dtype), _scale_head_grad(dw, g_total, ctx.w_dtype), None, None, None
+
+
+def _scale_head_grad(t: torch.Tensor, g: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """``t * g`` rounded to ``dtype`` in one pass.  The tensor library's product where autograd needs one that it can record
+    or batch: under ``create_graph``, and under ``is_grads_batched``, whose ``g`` has no storage."""
+    if torch.is_grad_enabled() or not torch._C._has_storage(g) or not t.is_cuda:
+        return (t * (g.to(t.dtype) if t.dtype == dtype else g)).to(dtype)
+    from . import lib, stream_ptr, _check
+    g = g.float().reshape(1)
+    out = torch.empty(t.shape, dtype=torch.bfloat16, device=t.device)
+    _check(lib().cm_scale_to_bf16(t.data_ptr(), int(t.dtype == torch.float32), out.data_ptr(), g.data_ptr(), t.numel(), stream_ptr()),
+           "cm_scale_to_bf16")
+    F_.count_launch("scale_to_bf16")
+    return out
 
 
 def linear_cross_entropy_weighted(h, w, labels, weights, ignore_index):

@@ -122,3 +122,17 @@ def test_linear_ce_chunk_and_vocabulary_edges(T, H, V):
     """A vocabulary of one vector, one that ends inside an unrolled group of vectors, and a last chunk of one row (the first
     chunk writes dw, the second adds to it)."""
     test_linear_ce_weighted(T, H, V)
+
+
+def test_linear_ce_batched_upstream_gradients():
+    """``is_grads_batched`` gives, slice by slice, the bits of one backward per upstream gradient."""
+    from cppmega_b200.ops.cuda import extra
+    torch.manual_seed(0)
+    h = torch.randn(70, 64, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(512, 64, device="cuda") * 0.1).bfloat16().requires_grad_()
+    total, _ = extra.linear_cross_entropy_weighted(h, w, torch.randint(0, 512, (70,), device="cuda"), torch.rand(70, device="cuda"), -100)
+    gs = torch.tensor([1.0, 0.37], device="cuda")
+    batched = torch.autograd.grad(total, [h, w], gs, is_grads_batched=True, retain_graph=True)
+    for i, g in enumerate(gs):
+        one = torch.autograd.grad(total, [h, w], g, retain_graph=True)
+        assert torch.equal(batched[0][i], one[0]) and torch.equal(batched[1][i], one[1])
