@@ -29,6 +29,17 @@ __device__ __forceinline__ uint8_t e8m0_from_amax(float amax) {
   e = e < 1 ? 1 : (e > 254 ? 254 : e);
   return (uint8_t)e;
 }
+// The same for a tensor-wide amax, which the caller may give as any fp32 value: the bits above differ from the definition's
+// logarithm, which rounds to k for the values closest above 448 * 2^k.
+__device__ __forceinline__ uint8_t e8m0_from_tensor_amax(float amax) {
+  if (!(amax > 0.f)) return 127;
+  if (isinf(amax)) return 1;
+  const int e = (int)ceilf(log2f(amax * (1.f / 448.f))) + 127;
+  return (uint8_t)(e < 1 ? 1 : (e > 254 ? 254 : e));
+}
+__device__ __forceinline__ uint8_t scale_byte(const float* tamax, float block_amax) {
+  return tamax ? e8m0_from_tensor_amax(*tamax) : e8m0_from_amax(block_amax);
+}
 // 2^(127 - sb), sb in 1..254
 __device__ __forceinline__ float inverse_scale(uint8_t sb) { return __uint_as_float(sb == 254 ? 0x00400000u : (254u - sb) << 23); }
 // two floats -> two e4m3 bytes (lo in bits 0..7)
@@ -72,7 +83,7 @@ __global__ void __launch_bounds__(256) quantize_rowwise_kernel(const __nv_bfloat
     const unsigned live = __activemask();          // whole groups of four threads enter or leave the loop together
     am = fmaxf(am, __shfl_xor_sync(live, am, 1));
     am = fmaxf(am, __shfl_xor_sync(live, am, 2));
-    const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
+    const uint8_t sb = scale_byte(tamax, am);
     const float mult = inverse_scale(sb);
     uint2 o;
     o.x = (uint32_t)to_e4m3x2(f[0] * mult, f[1] * mult) | ((uint32_t)to_e4m3x2(f[2] * mult, f[3] * mult) << 16);
@@ -102,7 +113,7 @@ __global__ void __launch_bounds__(128) quantize_colwise_kernel(const __nv_bfloat
     f[r] = (r0 + r < rows) ? __bfloat162float(x[(size_t)(r0 + r) * cols + c]) : 0.f;
     am = fmaxf(am, fabsf(f[r]));
   }
-  const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
+  const uint8_t sb = scale_byte(tamax, am);
   const float mult = inverse_scale(sb);
   uint32_t w[8];
 #pragma unroll
@@ -159,7 +170,7 @@ __global__ void __launch_bounds__(256) quantize_both_kernel(const __nv_bfloat16*
     w[0] = raw[it].x; w[1] = raw[it].y; w[2] = raw[it].z; w[3] = raw[it].w;
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
     am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
-    const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am);
+    const uint8_t sb = scale_byte(tamax, am);
     const float mult = inverse_scale(sb);
     if ((lane & 3) == 0) s_r[row][v >> 2] = sb;
     if (row < nrows && v * 8 < ncols) {
@@ -182,7 +193,7 @@ __global__ void __launch_bounds__(256) quantize_both_kernel(const __nv_bfloat16*
     }
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const uint8_t sb = e8m0_from_amax(tamax ? *tamax : am[h]);
+      const uint8_t sb = scale_byte(tamax, am[h]);
       const float mult = inverse_scale(sb);
       s_t[pair * 2 + h][blk] = sb;
       uint32_t o[8];

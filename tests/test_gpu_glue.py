@@ -490,6 +490,20 @@ def test_tensorwise_fp8_quantisers_and_linear():
     assert _rel(y.reshape(-1, 128), x2.float() @ w.detach().float().t()) < 6e-2
 
 
+@pytest.mark.parametrize("k", [-130, -20, 0, 1, 10, 20, 119])
+@pytest.mark.parametrize("ulps", [0, 1, 3, 8, 64])
+def test_tensorwise_scale_of_any_fp32_amax(k, ulps):
+    """A caller's amax need not be a bf16 value: just above 448 * 2^k the scale byte is the definition's, whose logarithm
+    rounds to k."""
+    from cppmega_b200.ops import reference as ref
+    from cppmega_b200.ops.cuda import mxfp8
+    am = (torch.tensor([448.0], dtype=torch.float64) * 2.0 ** k).float().view(torch.int32).add(ulps).view(torch.float32).cuda()
+    want = ref.e8m0_from_amax(am).item()
+    x = torch.randn(64, 96, device="cuda").bfloat16()
+    for q in (mxfp8.quantize_rowwise(x, tensorwise=am), mxfp8.quantize_colwise(x, tensorwise=am), *mxfp8.quantize_both(x, True, am)):
+        assert q.scales.unique().tolist() == [want]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("grad_dtype", [None, torch.float32, torch.bfloat16])
 def test_embedding_kernels_gather_and_scatter_add(grad_dtype):
