@@ -165,8 +165,10 @@ class LinearCEWeightedFn(torch.autograd.Function):
 
 def _scale_head_grad(t: torch.Tensor, g: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
     """``t * g`` rounded to ``dtype`` in one pass.  The tensor library's product where autograd needs one that it can record
-    or batch: under ``create_graph``, and under ``is_grads_batched``, whose ``g`` has no storage."""
-    if torch.is_grad_enabled() or not torch._C._has_storage(g) or not t.is_cuda:
+    or batch: under ``create_graph``, and under ``is_grads_batched``, whose ``g`` has no storage; and for a ``t`` that a
+    saved-tensor hook gave back in a layout or type the kernel does not read."""
+    if (torch.is_grad_enabled() or not torch._C._has_storage(g) or not t.is_cuda or not t.is_contiguous()
+            or t.dtype not in (torch.float32, torch.bfloat16) or t.data_ptr() % 16):
         return (t * (g.to(t.dtype) if t.dtype == dtype else g)).to(dtype)
     from . import lib, stream_ptr, _check
     g = g.float().reshape(1)

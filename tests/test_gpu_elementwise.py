@@ -136,3 +136,22 @@ def test_linear_ce_batched_upstream_gradients():
     for i, g in enumerate(gs):
         one = torch.autograd.grad(total, [h, w], g, retain_graph=True)
         assert torch.equal(batched[0][i], one[0]) and torch.equal(batched[1][i], one[1])
+
+
+@pytest.mark.parametrize("unpack", [lambda t: t.t().contiguous().t(),
+                                    lambda t: torch.cat([t.new_zeros(1), t.reshape(-1)])[1:].view(t.shape),
+                                    lambda t: t.double()])
+def test_linear_ce_gradients_given_back_in_another_form(unpack):
+    """A saved-tensor hook may return a transposed, an unaligned or a wider tensor of the same values: the gradients are those of the same
+    values saved plainly, to the one rounding in which a wider product differs."""
+    from cppmega_b200.ops.cuda import extra
+    torch.manual_seed(0)
+    h = torch.randn(72, 64, device="cuda").bfloat16().requires_grad_()
+    w = (torch.randn(512, 64, device="cuda") * 0.1).bfloat16().requires_grad_()
+    lab, rw, g = torch.randint(0, 512, (72,), device="cuda"), torch.rand(72, device="cuda"), torch.tensor(0.37, device="cuda")
+    plain = torch.autograd.grad(extra.linear_cross_entropy_weighted(h, w, lab, rw, -100)[0], [h, w], g)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: unpack(t) if t.is_floating_point() else t):
+        total = extra.linear_cross_entropy_weighted(h, w, lab, rw, -100)[0]
+        other = torch.autograd.grad(total, [h, w], g)
+    for a, b in zip(other, plain):
+        assert _rel(a, b) < 2.0 ** -8
