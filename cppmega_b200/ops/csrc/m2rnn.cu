@@ -5,14 +5,14 @@
 // One CTA per (batch, head), one warp per 16 rows of the state h [KD x 16], which stays in registers for the whole sequence
 // in the accumulator layout of mma.m16n8k16 (lane (g, t): rows g and g + 8, columns 2t, 2t + 1 of each 8-column half).  That
 // layout is also the A operand of the next step's product with W, so a step exchanges nothing between lanes.  The products
-// keep fp32 operands: W is bf16 as given, and the fp32 factor is the sum of three bf16 parts (8 + 8 + 8 mantissa bits), each
-// multiplied exactly and added in fp32.
+// keep fp32 operands: a bf16 factor enters as it is, an fp32 one as the sum of three bf16 parts (8 + 8 + 8 mantissa bits), each
+// multiplied exactly and added in fp32; of the nine products of two such factors those below 2^-24 are left out.
 //
 // What bounds it: the instructions of a step - one warp per scheduler, each instruction 2.3 cycles at the dependences of a chain -
 // not arithmetic or memory.  So every sum that can be one is a matrix product: the gradients of k and q against an operand
 // with v and dy in two of its columns, the gradient of v against one with k in a row.  With four
 // threads per row, 12 shuffles and 64 dependent multiply-adds a step and the state history fetched one step ahead, the
-// backward took 1.23 us and the forward 0.29 us a step at batch 2, 51 heads; now 0.44 and 0.26 (1,788 us and 1,082 us in all).
+// backward took 1.23 us and the forward 0.29 us a step at batch 2, 51 heads; now 0.45 and 0.26.
 // The history is requested four steps ahead.  Two warps per 16 rows, the second forming the gradients a block of steps behind,
 // were slower (0.61 us a step: 589 instructions between them instead of 378 then in one warp).
 // Only dh_{t-1} = f_t dh_t + da_t W^T is on the backward's chain; the replay of tanh(a_t) and all other gradients hang off it.
@@ -279,8 +279,12 @@ struct BwdShared {
   float dw[VD][VD];
 };
 
+// One resident CTA is asked for, so that the compiler keeps a step's independent products apart in up to 255 registers: left to
+// choose, it takes 182 and 602 us for 1,024 steps of 102 heads, against 511 (16 and 32 rows: 639 and 596 against 501 and 513).
+// Calls of more CTAs than fit at two an SM lose by it (1,351 -> 1,212 us at 408 of them, 1,012 with the 167 registers and the
+// lower precision of two parts).
 template <int KD>
-__global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
+__global__ void __launch_bounds__(KD * 2, 1) m2rnn_bwd_kernel(
     const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
     const __nv_bfloat16* __restrict__ W, const float* __restrict__ f, const float* __restrict__ hist,
     const __nv_bfloat16* __restrict__ dy, float* __restrict__ dq_h, float* __restrict__ dk_h,
@@ -367,11 +371,6 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
     if (blk > 0) in.fetch((blk - 1) * TB, tid);
     if (blk + 1 < nblocks) write_out(blk + 1);
     const int t0 = blk * TB;
-    float dw_blk[2][4];                           // this block's part of dW: added to the running sum once per block
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) dw_blk[n][i] = 0.f;
 #pragma unroll 1
     for (int t1 = TB - AHEAD; t1 >= 0; t1 -= AHEAD) {
 #pragma unroll
@@ -427,25 +426,33 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
           }
         }
         // dW[u][v] += sum_rows h_{t-1}[row][u] da[row][v] and dv[v] = sum_rows k[row] da[row][v]: da as the right factor, h as the
-        // left one, both transposed within the warp.  Two parts of each (16 mantissa bits; k is exact): the sums are rounded to bf16.
+        // left one, both transposed within the warp.  All parts of both factors, down to the products of 2^-24 (k is exact); a
+        // step's sum starts from zero and is added to the running one in fp32 rounding.
         {
-          uint32_t hh[4], hm[4], dd[4], dm[4];
+          uint32_t hh[4], hm[4], hl[4], dd[4], dm[4], dl[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int j = (i & 1) * 2 + (i >> 1);  // block (row half, column half) -> (column half, row half)
-            hh[j] = transpose8x8(sp.hi[i]); hm[j] = transpose8x8(sp.mid[i]);
-            dd[i] = transpose8x8(sd.hi[i]); dm[i] = transpose8x8(sd.mid[i]);
+            hh[j] = transpose8x8(sp.hi[i]); hm[j] = transpose8x8(sp.mid[i]); hl[j] = transpose8x8(sp.lo[i]);
+            dd[i] = transpose8x8(sd.hi[i]); dm[i] = transpose8x8(sd.mid[i]); dl[i] = transpose8x8(sd.lo[i]);
           }
           const uint32_t kr[4] = {st.kb[t][warp * 8 + t4] & row0_mask, 0u, st.kb[t][warp * 8 + 4 + t4] & row0_mask, 0u};
           float dvp[2][4];
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
-            const uint32_t bh[2] = {dd[n * 2], dd[n * 2 + 1]}, bm[2] = {dm[n * 2], dm[n * 2 + 1]};
-            mma16816(dvp[n], kr, bm);
-            mma16816(dw_blk[n], hm, bh, dw_blk[n]);
+            const uint32_t bh[2] = {dd[n * 2], dd[n * 2 + 1]}, bm[2] = {dm[n * 2], dm[n * 2 + 1]}, bl[2] = {dl[n * 2], dl[n * 2 + 1]};
+            float dwp[4];
+            mma16816(dvp[n], kr, bl);
+            mma16816(dwp, hl, bh);
+            mma16816(dvp[n], kr, bm, dvp[n]);
+            mma16816(dwp, hh, bl, dwp);
             mma16816(dvp[n], kr, bh, dvp[n]);
-            mma16816(dw_blk[n], hh, bm, dw_blk[n]);
-            mma16816(dw_blk[n], hh, bh, dw_blk[n]);
+            mma16816(dwp, hm, bm, dwp);
+            mma16816(dwp, hm, bh, dwp);
+            mma16816(dwp, hh, bm, dwp);
+            mma16816(dwp, hh, bh, dwp);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dw_sum[n][i] += dwp[i];
           }
           if (g == 0) {
             *reinterpret_cast<float2*>(&sh.dv[p][t][warp][2 * t4]) = make_float2(dvp[0][0], dvp[0][1]);
@@ -456,10 +463,6 @@ __global__ void __launch_bounds__(KD * 2) m2rnn_bwd_kernel(
         hcur = sp;
       }
     }
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) dw_sum[n][i] += dw_blk[n][i];
     if (blk > 0) in.commit(sh.stage[(blk - 1) & 1], tid);
   }
   __syncthreads();

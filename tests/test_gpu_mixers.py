@@ -225,6 +225,34 @@ def test_m2rnn_blocks_and_unaligned_inputs(B, S, H, KD, shared, offset):
             assert a.grad.norm() == 0, name
 
 
+@pytest.mark.parametrize("B,S,KD", [(1, 1, 64), (1, 16, 16), (1, 16, 32), (2, 16, 64), (1, 19, 64)])
+def test_m2rnn_gradients_of_v_and_w_keep_fp32_factors(B, S, KD):
+    """dv and dW in fp32, before their rounding, against 64-bit sums of the kernel's own states and da.  With v the j-th unit
+    vector in head j, dk is the j-th column of da, exactly.  A few fp32 roundings of 2^-24 give up to 2e-7 here; factors cut
+    to two bf16 parts 1e-6 to 4e-6."""
+    from cppmega_b200.ops import cuda as cu
+    torch.manual_seed(S + KD)
+    H = 16
+    bf = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    q, k, dy = bf(B, S, H, KD), bf(B, S, H, KD), bf(B, S, H, 16)
+    v = torch.eye(16, device="cuda").bfloat16().expand(B, S, 16, 16).contiguous()
+    W = (torch.eye(16, device="cuda") + 0.1 * torch.randn(H, 16, 16, device="cuda")).bfloat16().contiguous()
+    f32 = lambda *s: torch.empty(*s, device="cuda")  # noqa: E731
+    f, y, hist = torch.rand(B, S, H, device="cuda"), torch.empty_like(dy), f32(B, H, S, KD, 16)
+    dq, dk, dv, df, dW = f32(B, S, H, KD), f32(B, S, H, KD), f32(B, S, H, 16), f32(B, S, H), torch.zeros(H, 16, 16, device="cuda")
+    ptr = lambda *ts: [t.data_ptr() for t in ts]  # noqa: E731
+    dims = (B, S, H, H, H, KD, 16, cu.stream_ptr())
+    assert cu.lib().cm_m2rnn_fwd(*ptr(q, k, v, W, f, y, hist), None, *dims) == 0
+    assert cu.lib().cm_m2rnn_bwd(*ptr(q, k, v, W, f, hist, dy, dq, dk, dv, df, dW), *dims) == 0
+    before = torch.zeros_like(hist)
+    before[:, :, 1:] = hist[:, :, :-1]
+    da, j = dk.double(), torch.arange(16)
+    err = lambda a, b: ((a - b).norm() / b.norm().clamp_min(1e-30)).item()  # noqa: E731
+    assert err(dv.double()[:, :, j, j], (k.double() * da).sum(-1)) < 2.0 ** -21
+    assert err(dW.double()[j, :, j], torch.einsum("bhsku,bshk->hu", before.double(), da)) < 2.0 ** -21
+    assert err(dq.double(), torch.einsum("bhskv,bshv->bshk", hist.double(), dy.double())) < 2.0 ** -21
+
+
 @pytest.mark.parametrize("B,S,H,std,scale", [(1, 128, 1, 0.7, 0.09), (1, 384, 2, 4.0, 0.09), (2, 640, 1, 0.7, -0.05), (1, 256, 3, 0.7, 0.0)])
 def test_dense_causal_attention_tile_pairs(B, S, H, std, scale):
     """Odd and even counts of query tiles (the last pair has one or two), scores large enough that the running maximum grows
