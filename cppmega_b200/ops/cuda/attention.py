@@ -72,6 +72,8 @@ def causal_attention(q, k, v, scale: float):
     if not supported(q, k, v):
         F_._miss("causal_attention(shape/dtype)", q)
         return F_.causal_attention_library(q, k, v, scale)
+    if scale < 0:       # the kernel takes the largest raw score of a row for its softmax reference: fold the sign into q, exactly
+        q, scale = -q, -scale
     return CausalAttentionFn.apply(q, k, v, float(scale))
 
 
