@@ -303,7 +303,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             tmem_ld_wait();
             const int col = t.n0 + c;
             if (row >= args.M) continue;
-            if (col + 32 <= args.N && (args.ldc % 8) == 0) {
+            if (col + 32 <= args.N && args.c_vec) {
               if constexpr (sizeof(OutT) == 2) {
                 uint4* dst = reinterpret_cast<uint4*>(crow + col);
 #pragma unroll
@@ -424,7 +424,9 @@ int launch_gemm_pair(int mode, bool a_mn, bool b_mn, bool out_fp32, const void* 
     rc = b_mn ? make_tmap_2d_bf16(&tmB, B, k_rows, args.N, ldb, 64) : make_tmap_2d_bf16(&tmB, B, args.N, args.K, ldb, half);
   if (rc) return rc;
   const int es = out_fp32 ? 4 : 2;
-  args.tma_store = !args.accumulate && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && (args.ldc * es) % 16 == 0;
+  const bool c_aligned = (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+  args.tma_store = !args.accumulate && c_aligned && (args.ldc * es) % 16 == 0;
+  args.c_vec = c_aligned && args.ldc % 8 == 0;
   if (args.tma_store) {
     rc = pair2::make_store_map(&tmC, C, out_fp32, mode == PAIR_GROUPED_K, args);
     if (rc) return rc;

@@ -56,6 +56,7 @@ struct PairArgs {
   const int* tile_expert;
   const int* seg_offsets;
   int* err;
+  int c_vec;               // rows of C start on 16-byte boundaries; set at the launch like tma_store
 };
 
 // A, B as in cm_gemm_bf16 / cm_grouped_gemm_*; returns 0 or an error code.

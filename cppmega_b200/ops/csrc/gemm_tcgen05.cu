@@ -80,6 +80,7 @@ struct GemmArgs {
   int my_slot;             // PEER_C: staging slot this rank writes on every peer
   long long local_rows;    // PEER_C: rows of one staging slot (= batch * rows_per_seg)
   void* c_peers[MAX_TP_PEERS];   // PEER_C: staging buffers [n_peers slots, local_rows, N]
+  int c_vec;               // rows of C start on 16-byte boundaries; set at the launch
 };
 
 template <int BN>
@@ -299,7 +300,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tmem_ld_wait();
         const int col = n0 + c * 32;
         if (!row_ok || col >= args.N) continue;
-        if (col + 32 <= args.N && (args.ldc % 8) == 0) {
+        if (col + 32 <= args.N && args.c_vec) {
           if constexpr (sizeof(OutT) == 2) {
             uint4* dst = reinterpret_cast<uint4*>(crow + col);
 #pragma unroll
@@ -428,6 +429,15 @@ int sm_count() {
   return n;
 }
 
+// The epilogue moves 16 bytes at a time where every row of C allows it, single elements elsewhere.
+static GemmArgs with_store_width(const GemmArgs& args, const void* C) {
+  GemmArgs a = args;
+  uintptr_t bits = reinterpret_cast<uintptr_t>(C);
+  for (int p = 0; p < MAX_TP_PEERS; ++p) bits |= reinterpret_cast<uintptr_t>(a.c_peers[p]);
+  a.c_vec = (bits & 15) == 0 && a.ldc % 8 == 0;
+  return a;
+}
+
 template <int BN, bool A_MN, bool B_MN, typename OutT, bool ACC, int MODE>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, OutT* C, const GemmArgs& args, int total_tiles,
                   cudaStream_t stream) {
@@ -440,7 +450,7 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, OutT* C, const
   }
   int grid = total_tiles < sm_count() ? total_tiles : sm_count();
   if (grid <= 0) return 0;
-  kern<<<grid, GEMM_THREADS, SmemLayout<BN>::TOTAL, stream>>>(tmA, tmB, C, args, NoPeerMaps{});
+  kern<<<grid, GEMM_THREADS, SmemLayout<BN>::TOTAL, stream>>>(tmA, tmB, C, with_store_width(args, C), NoPeerMaps{});
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -456,7 +466,7 @@ static int launch_peer_a(const PeerMaps& pm, const CUtensorMap& tmB, __nv_bfloat
   }
   int grid = total_tiles < sm_count() ? total_tiles : sm_count();
   if (grid <= 0) return 0;
-  kern<<<grid, GEMM_THREADS, SmemLayout<BN>::TOTAL, stream>>>(pm.m[0], tmB, C, args, pm);
+  kern<<<grid, GEMM_THREADS, SmemLayout<BN>::TOTAL, stream>>>(pm.m[0], tmB, C, with_store_width(args, C), pm);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -643,7 +653,7 @@ static int launch_peer_k(const PeerMaps& pm, const CUtensorMap& tmA, const CUten
   }
   int grid = total_tiles < sm_count() ? total_tiles : sm_count();
   if (grid <= 0) return 0;
-  kern<<<grid, GEMM_THREADS, SmemLayout<BN>::TOTAL, stream>>>(tmA, tmB, C, args, pm);
+  kern<<<grid, GEMM_THREADS, SmemLayout<BN>::TOTAL, stream>>>(tmA, tmB, C, with_store_width(args, C), pm);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

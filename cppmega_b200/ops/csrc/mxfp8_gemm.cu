@@ -57,6 +57,7 @@ struct Args {
   const int* seg_offsets;    // GROUPED_K: [E + 1], multiples of 128
   int num_experts;
   int b_row_e, b_k_e;        // GROUPED_ROWS: row / column offset of expert e in B is e * b_row_e / e * b_k_e (multiples of 128)
+  int c_vec;                 // rows of C start on 16-byte boundaries: the epilogue moves 16 bytes at a time, else single elements
 };
 
 struct Tile {
@@ -103,7 +104,7 @@ template <typename OutT, bool ACC>
 __device__ __forceinline__ void store_rows(OutT* __restrict__ C, const Args& args, const uint32_t (&r)[4][32], int row, int col0, int e) {
   if (row >= args.M || col0 >= args.N) return;
   OutT* crow = C + (long long)e * args.M * args.ldc + (long long)row * args.ldc + col0;
-  if (col0 + 128 <= args.N && (args.ldc % 8) == 0) {
+  if (col0 + 128 <= args.N && args.c_vec) {
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       if constexpr (sizeof(OutT) == 2) {
@@ -557,6 +558,12 @@ static int make_tmap_sf(CUtensorMap* out, const void* base, uint64_t tiles) {
   return r == CUDA_SUCCESS ? 0 : int(r);
 }
 
+static Args with_store_width(const Args& args, const void* C) {
+  Args a = args;
+  a.c_vec = (reinterpret_cast<uintptr_t>(C) & 15) == 0 && a.ldc % 8 == 0;
+  return a;
+}
+
 template <typename OutT, bool ACC>
 static int launch_pair(const void* A, const void* B, void* C, long long lda, long long ldb, const Args& args, int tiles, cudaStream_t s) {
   CUtensorMap tmA, tmB, tmSA, tmSB;
@@ -571,7 +578,8 @@ static int launch_pair(const void* A, const void* B, void* C, long long lda, lon
     attr_set.done();
   }
   const int pairs = sm_count() / 2;
-  kern<<<2 * (tiles < pairs ? tiles : pairs), THREADS, mxpair::SMEM_TOTAL, s>>>(tmA, tmB, tmSA, tmSB, reinterpret_cast<OutT*>(C), args);
+  kern<<<2 * (tiles < pairs ? tiles : pairs), THREADS, mxpair::SMEM_TOTAL, s>>>(tmA, tmB, tmSA, tmSB, reinterpret_cast<OutT*>(C),
+                                                                                               with_store_width(args, C));
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -586,7 +594,7 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, const
   const int tiles = ((args.M + BM - 1) / BM) * ((args.N + BN - 1) / BN) * (MODE == GROUPED_K ? args.num_experts : 1);
   const int grid = tiles < sm_count() ? tiles : sm_count();
   if (grid <= 0) return 0;
-  kern<<<grid, THREADS, SMEM_TOTAL, s>>>(tmA, tmB, reinterpret_cast<OutT*>(C), args);
+  kern<<<grid, THREADS, SMEM_TOTAL, s>>>(tmA, tmB, reinterpret_cast<OutT*>(C), with_store_width(args, C));
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

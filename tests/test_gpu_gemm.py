@@ -156,3 +156,45 @@ def test_grouped_experts_pair_tiles(cu, counts):
     yr.backward(g.float())
     for got, want in ((y, yr), (x.grad, xr.grad), (w1.grad, w1r.grad), (w2.grad, w2r.grad)):
         assert _rel(got, want) < 1.5e-2
+
+
+@pytest.mark.parametrize("pair,bn", [(1, 256), (1, 128), (0, 128), (0, 64)])
+@pytest.mark.parametrize("offset,pitch", [(1, 264), (4, 264), (8, 264), (0, 257), (2, 260)])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.bfloat16, True), (torch.float32, True)])
+def test_gemm_result_in_an_unaligned_view(cu, pair, bn, offset, pitch, out, accumulate):
+    """C starts off a 16-byte boundary, or its rows do: every element is still written, and nothing beside it.  Tolerances as
+    for aligned results (test_gemm_tile_shapes)."""
+    M, N, K = 200, 256, 136
+    torch.manual_seed(offset + pitch)
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, K, device="cuda").bfloat16()
+    buf = torch.randn(offset + M * pitch, device="cuda").to(out)
+    before = buf.clone()
+    C, C0 = (t[offset:].view(M, pitch)[:, :N] for t in (buf, before))
+    rc = cu.lib().cm_gemm_bf16_tiled(a.data_ptr(), b.data_ptr(), C.data_ptr(), M, N, K, K, K, pitch, 0, 0, int(out == torch.float32),
+                                     int(accumulate), pair, bn, cu.err_word(a.device).data_ptr(), cu.stream_ptr())
+    assert rc == 0
+    cu.check_errors()
+    ref = a.double() @ b.double().t() + (C0.double() if accumulate else 0)
+    assert ((C.double() - ref).norm() / ref.norm()).item() < (1e-5 if out == torch.float32 else 4e-3)
+    C.copy_(C0)
+    assert torch.equal(buf, before)
+
+
+@pytest.mark.parametrize("M", [96, 288])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, True)])
+def test_mxfp8_gemm_result_in_an_unaligned_view(cu, M, out, accumulate):
+    """The same for the block-scaled GEMM, on one CTA (M <= 128) and on a CTA pair or one CTA (M > 128)."""
+    from cppmega_b200.ops.cuda import mxfp8
+    torch.manual_seed(M)
+    N, K = 160, 96
+    a, b = (mxfp8.quantize_rowwise(torch.randn(r, K, device="cuda").bfloat16()) for r in (M, N))
+    for offset, pitch in ((1, 168), (0, 163)):
+        buf = torch.randn(offset + M * pitch, device="cuda").to(out)
+        before = buf.clone()
+        C, C0 = (t[offset:].view(M, pitch)[:, :N] for t in (buf, before))
+        mxfp8.gemm_mxfp8(a, b, out=C, accumulate=accumulate)
+        cu.check_errors()
+        ref = mxfp8.dequantize(a).double() @ mxfp8.dequantize(b).double().t() + (C0.double() if accumulate else 0)
+        assert ((C.double() - ref).norm() / ref.norm()).item() < (1e-5 if out == torch.float32 else 4e-3)
+        C.copy_(C0)
+        assert torch.equal(buf, before)
