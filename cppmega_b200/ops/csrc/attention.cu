@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_kernel(const __grid_c
   uint8_t* sQ = smem;                      // 2 query tiles [128 x 128]
   uint8_t* sKV = sQ + 4 * SLAB;            // stages of K [128 x 128], V [128 x 64]
   FwdShared* sh = reinterpret_cast<FwdShared*>(sKV + KV_STAGES * 3 * SLAB);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
 
   // pairs with many key tiles first
   const int n_pairs = (a.n_qt + 1) >> 1;
@@ -150,9 +149,13 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_kernel(const __grid_c
   }
   if (warp == 8) { tmem_alloc(&sh->tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = sh->tmem_slot;     // S_t at 128 t, O_t at 256 + 64 t, P_t at 384 + 64 t
+  if (drain) {
+    if (warp == 8) tmem_dealloc(tmem, 512);
+    return;
+  }
 
   if (warp == 9) {
     // ------------------------------ TMA producer ------------------------------
@@ -424,7 +427,6 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   uint8_t* sdS = sP + 2 * SLAB;
   uint8_t* sdQ = sdS + 2 * SLAB;            // 4 warps x [32 queries x 32 fp32], 128-byte-swizzled
   BwdShared* sh = reinterpret_cast<BwdShared*>(sdQ + SLAB);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
 
   int bh, kt;                               // key tile 0 has the longest loop
   decode_cta(blockIdx.x, a.n_kt, gridDim.x / a.n_kt, a.heads_per_group, bh, kt);
@@ -450,9 +452,13 @@ __global__ void __launch_bounds__(BWD_THREADS, 1) attn_bwd_kernel(const __grid_c
   }
   if (warp == 12) { tmem_alloc(&sh->tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = sh->tmem_slot;
+  if (drain) {
+    if (warp == 12) tmem_dealloc(tmem, 512);
+    return;
+  }
   const uint32_t tS = tmem, tdP = tmem + 128, tdV = tmem + 256, tdK = tmem + 320, tdQ = tmem + 448;
   const uint32_t lane_addr = uint32_t((warp & 3) * 32) << 16;
   const int row0 = b * a.S;

@@ -104,6 +104,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The set-up barrier of a block.  True in every thread if the error word was set when the block started (an earlier kernel or
+// another block gave up): the block frees what it has set up and leaves as one.  Read by each thread for itself, the word could
+// send some warps away and leave others with barriers and a TMEM address that nobody wrote.
+__device__ __forceinline__ bool setup_barrier(const int* err) {
+  return __syncthreads_or(threadIdx.x == 0 && err && *reinterpret_cast<const volatile int*>(err) != 0);
+}
+
 // ---- cross-GPU flags ------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long global_timer_ns() {
   unsigned long long t;

@@ -108,7 +108,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  if (args.err && *reinterpret_cast<volatile int*>(args.err) != 0) return;   // an earlier kernel gave up: drain
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
@@ -135,9 +134,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(args.err);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (drain) {
+    if (warp == 1) tmem_dealloc(tmem_base, 2 * BN);
+    return;
+  }
 
   // tile -> (expert, m0, n0, first k block, number of k blocks); identical in every role
   auto decode = [&](int tile, int& e, int& m0, int& n0, int& kb0, int& nkb) {

@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(THREADS, 2) head_linear_kernel(const __grid_co
   uint8_t* sX = smem;                       // 2 stages
   uint8_t* sW = sX + 2 * SLAB;              // 2 stages
   Shared* sh = reinterpret_cast<Shared*>(sW + 2 * WSLAB);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
   const int tid = threadIdx.x, warp = tid >> 5;
   const int t0 = blockIdx.x * BT;
   if (tid == 0) {
@@ -71,9 +70,13 @@ __global__ void __launch_bounds__(THREADS, 2) head_linear_kernel(const __grid_co
   }
   if (warp == 0) { tmem_alloc(&sh->tmem_slot, 128); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = sh->tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 128);
+    return;
+  }
   const uint32_t lane_addr = uint32_t((warp & 3) * 32) << 16;
   volatile int* abort_flag = &sh->abort_flag;
   constexpr uint32_t idesc = umma_idesc_bf16(BT, HD, false, B_MN);
@@ -157,7 +160,6 @@ __global__ void __launch_bounds__(THREADS, 1) head_linear_wgrad_kernel(const __g
   uint8_t* sA = smem;                       // 2 stages x [dy_h0 | dy_h1]
   uint8_t* sB = sA + 4 * SLAB;              // 2 stages x [x_h0 | x_h1]
   Shared* sh = reinterpret_cast<Shared*>(sB + 4 * SLAB);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
   const int tid = threadIdx.x, warp = tid >> 5;
   const int hp = blockIdx.x, split = blockIdx.y;
   const int n_tiles_all = (a.T + BT - 1) / BT;
@@ -171,9 +173,13 @@ __global__ void __launch_bounds__(THREADS, 1) head_linear_wgrad_kernel(const __g
   }
   if (warp == 0) { tmem_alloc(&sh->tmem_slot, 128); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = sh->tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 128);
+    return;
+  }
   const uint32_t lane_addr = uint32_t((warp & 3) * 32) << 16;
   volatile int* abort_flag = &sh->abort_flag;
   constexpr uint32_t idesc = umma_idesc_bf16(128, 128, true, true);

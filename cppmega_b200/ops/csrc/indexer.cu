@@ -48,7 +48,6 @@ __global__ void __launch_bounds__(128) indexer_scores_kernel(const __grid_consta
   uint8_t* sQ = smem;
   uint8_t* sK = smem + SLAB;
   ScoreShared* sh = reinterpret_cast<ScoreShared*>(sK + STAGES * SLAB);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
   const int b = blockIdx.y;
   const int qt = gridDim.x - 1 - blockIdx.x;                   // long rows first
   const int i0 = qt * QT;
@@ -66,9 +65,13 @@ __global__ void __launch_bounds__(128) indexer_scores_kernel(const __grid_consta
   }
   if (warp == 0) { tmem_alloc(&sh->tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = sh->tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 256);
+    return;
+  }
   const uint32_t lane_addr = uint32_t(warp * 32) << 16;
   volatile int* abort_flag = &sh->abort_flag;
   const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK);

@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(THREADS2) mimo_grad_state_kernel(const __grid_
   uint64_t* bars = reinterpret_cast<uint64_t*>(sc + 1);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;   // an earlier CTA / kernel gave up: drain
   int b, g, c, h;
   decode_block_b(a, b, g, c, h);
   const int t0 = c * LT;
@@ -152,9 +151,13 @@ __global__ void __launch_bounds__(THREADS2) mimo_grad_state_kernel(const __grid_
   }
   if (warp == 0) { tmem_alloc(tmem_slot, 64); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 64);
+    return;
+  }
   if (threadIdx.x == 0) {
     mbar_expect_tx(&bars[0], QT);
 #pragma unroll
@@ -274,7 +277,6 @@ __global__ void __launch_bounds__(THREADS2, 1) mimo_chunk_grad_kernel(const __gr
   // (biases die before phase A writes Pm; the scratch is used only after phase 2 has read it)
   static_assert(sizeof(GradScratch) <= 2 * SLAB && sizeof(HeadBias<N>) <= 2 * SLAB, "scratch must fit the Pm tile");
 
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;   // an earlier CTA / kernel gave up: drain
   const int tid = threadIdx.x;
   const int i = tid & 127, wg = tid >> 7, t = i >> 2, r = i & 3, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
@@ -284,9 +286,13 @@ __global__ void __launch_bounds__(THREADS2, 1) mimo_chunk_grad_kernel(const __gr
   }
   if (warp == 0) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 512);
+    return;
+  }
   // Persistent: one CTA per SM walks the chunks with a grid stride; barriers, TMEM and the kernel prologue are paid
   // once, and every barrier completes exactly one phase per chunk, so its parity is the iteration's low bit.
   uint32_t par = 0;

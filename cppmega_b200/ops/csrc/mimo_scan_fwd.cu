@@ -96,7 +96,6 @@ __global__ void __launch_bounds__(THREADS2) mimo_local_state_kernel(const __grid
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;   // an earlier CTA / kernel gave up: drain
   int b, g, c, h;
   decode_block(a, b, g, c, h);
   const int t0 = c * LT;
@@ -116,9 +115,13 @@ __global__ void __launch_bounds__(THREADS2) mimo_local_state_kernel(const __grid
   }
   if (warp == 0) { tmem_alloc(tmem_slot, 64); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 64);
+    return;
+  }
   if (threadIdx.x == 0) {
     mbar_expect_tx(&bars[0], KT);
 #pragma unroll
@@ -218,7 +221,6 @@ __global__ void __launch_bounds__(THREADS2, 2) mimo_chunk_out_kernel(const __gri
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;   // an earlier CTA / kernel gave up: drain
   int b, g, c, h;
   decode_block(a, b, g, c, h);
   const int t0 = c * LT;
@@ -242,9 +244,13 @@ __global__ void __launch_bounds__(THREADS2, 2) mimo_chunk_out_kernel(const __gri
   }
   if (warp == 0) { tmem_alloc(tmem_slot, 256); tmem_relinquish(); }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 256);
+    return;
+  }
   const uint32_t tS1 = tmem, tO2 = tmem + 128, tO1 = tmem + 192;
   if (threadIdx.x == 0) {
     mbar_expect_tx(&bars[0], 2 * QT + N * 128);

@@ -174,7 +174,6 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_empty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  if (args.err && *reinterpret_cast<volatile int*>(args.err) != 0) return;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int tiles_n = (args.N + BN - 1) / BN;
@@ -198,9 +197,13 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(args.err);
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (drain) {
+    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+    return;
+  }
 
   auto decode = [&](int tile) {
     Tile t;

@@ -78,7 +78,6 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_fwd_kernel(const __grid
   uint8_t* sP = sKV + 4 * SLAB;              // 2 key tiles x [128 keys x 64 heads]
   uint8_t* sQ = sP + 2 * SLAB;               // 2 dim slabs x [32 heads x 64]
   Shared* sh = reinterpret_cast<Shared*>(sQ + 2 * HQ * 128);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
 
   const long long token = blockIdx.x;
   const int b = (int)(token / a.S);
@@ -100,10 +99,14 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_fwd_kernel(const __grid
     for (int cc = 4; cc < 8; ++cc) *reinterpret_cast<uint4*>(sP + wg * SLAB + sw_off(i, cc)) = z;
   }
   tc_fence_before();
-  __syncthreads();                             // barriers initialised, TMEM address and key indices published
+  const bool drain = setup_barrier(a.err);     // barriers initialised, TMEM address and key indices published
   tc_fence_after();
-  gather_rows(sKV, a.kv + (size_t)b * a.Skv * D, sh->kidx, tid);
   const uint32_t tmem = sh->tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 128);
+    return;
+  }
+  gather_rows(sKV, a.kv + (size_t)b * a.Skv * D, sh->kidx, tid);
   const uint32_t tS = tmem, tO = tmem + 64;
   const uint32_t lane_addr = uint32_t((warp & 3) * 32) << 16;
   volatile int* abort_flag = &sh->abort_flag;
@@ -256,7 +259,6 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_bwd_kernel(const __grid
   uint8_t* sA = sKV + 4 * SLAB;              // 2 key tiles x [128 keys x (32 dS | 32 P)]
   uint8_t* sB = sA + 2 * SLAB;               // 2 dim slabs x [64 rows x 64]: rows 0..31 Q, rows 32..63 (dO | 0)
   BwdShared* sh = reinterpret_cast<BwdShared*>(sB + 2 * 64 * 128);
-  if (a.err && *reinterpret_cast<volatile int*>(a.err) != 0) return;
 
   const long long token = blockIdx.x;
   const int b = (int)(token / a.S);
@@ -290,9 +292,13 @@ __global__ void __launch_bounds__(THREADS, 2) sparse_mla_bwd_kernel(const __grid
     }
   }
   tc_fence_before();
-  __syncthreads();
+  const bool drain = setup_barrier(a.err);
   tc_fence_after();
   const uint32_t tmem = sh->tmem_slot;
+  if (drain) {
+    if (warp == 0) tmem_dealloc(tmem, 256);
+    return;
+  }
   gather_rows(sKV, a.kv + (size_t)b * a.Skv * D, sh->kidx, tid);
   const uint32_t tS = tmem, tdP = tmem + 64, tdQ = tmem, tdKV = tmem + 128;
   const uint32_t lane_addr = uint32_t((warp & 3) * 32) << 16;
