@@ -510,7 +510,7 @@ static DensePlan plan_dense(int M, int N, bool b_mn) {
   return best;
 }
 
-// cm_gemm_bf16 with the tile shape given: pair = 1: bn 128 or 256, with a K-major B also 192; pair = 0: bn 64 or 128.
+// cm_gemm_bf16 with the tile shape given: pair = 1: bn 128 or 256, with a K-major B also 192; pair = 0: bn 64, 128 or 256.
 extern "C" int cm_gemm_bf16_tiled(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                                   long long ldc, int a_mn, int b_mn, int out_fp32, int accumulate, int pair, int bn, int* err,
                                   cudaStream_t stream) {
@@ -522,7 +522,7 @@ extern "C" int cm_gemm_bf16_tiled(const void* A, const void* B, void* C, int M, 
     const PairArgs args{M, N, K, bn, ldc, 1, accumulate, 0, nullptr, nullptr, err};
     return launch_gemm_pair(PAIR_DENSE, a_mn, b_mn, out_fp32, A, B, C, lda, ldb, K, args, stream);
   }
-  if (bn != 64 && bn != 128) return -10;
+  if (bn != 64 && bn != 128 && bn != 256) return -10;
   CUtensorMap tmA, tmB;
   int rc = a_mn ? make_tmap_2d_bf16(&tmA, A, K, M, lda, 64) : make_tmap_2d_bf16(&tmA, A, M, K, lda, BM);
   if (rc) return rc;
@@ -531,8 +531,9 @@ extern "C" int cm_gemm_bf16_tiled(const void* A, const void* B, void* C, int M, 
   GemmArgs args{M, N, K, ldc, 1, nullptr, nullptr, err, 0, 0, 0, 0, {}};
   const int tiles = ((M + BM - 1) / BM) * ((N + bn - 1) / bn);
 #define CM_DENSE(OUT, ACC_)                                                                                          \
-  (bn == 64 ? dispatch_layout<64, OUT, ACC_, DENSE>(a_mn, b_mn, tmA, tmB, (OUT*)C, args, tiles, stream)               \
-            : dispatch_layout<128, OUT, ACC_, DENSE>(a_mn, b_mn, tmA, tmB, (OUT*)C, args, tiles, stream))
+  (bn == 64    ? dispatch_layout<64, OUT, ACC_, DENSE>(a_mn, b_mn, tmA, tmB, (OUT*)C, args, tiles, stream)            \
+   : bn == 128 ? dispatch_layout<128, OUT, ACC_, DENSE>(a_mn, b_mn, tmA, tmB, (OUT*)C, args, tiles, stream)           \
+               : dispatch_layout<256, OUT, ACC_, DENSE>(a_mn, b_mn, tmA, tmB, (OUT*)C, args, tiles, stream))
   if (out_fp32) return accumulate ? CM_DENSE(float, true) : CM_DENSE(float, false);
   return accumulate ? CM_DENSE(__nv_bfloat16, true) : CM_DENSE(__nv_bfloat16, false);
 #undef CM_DENSE

@@ -103,9 +103,11 @@ def _check(rc: int, what: str) -> None:
 # ---------------------------------------------------------------------------
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
-         out: Optional[torch.Tensor] = None, out_dtype=torch.bfloat16, accumulate: bool = False) -> torch.Tensor:
+         out: Optional[torch.Tensor] = None, out_dtype=torch.bfloat16, accumulate: bool = False,
+         peer_out: bool = False) -> torch.Tensor:
     """``C[M,N] = op(A) op(B)``.  ``a`` is [M,K] (or [K,M] when ``a_mn``); ``b`` is [N,K] (or [K,N]
-    when ``b_mn``).  bf16 inputs, fp32 accumulation in TMEM, bf16 or fp32 output."""
+    when ``b_mn``).  bf16 inputs, fp32 accumulation in TMEM, bf16 or fp32 output.  ``peer_out``: ``out`` lies in another
+    GPU's memory; the one-CTA kernel writes it with ordinary stores."""
     assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
     assert a.stride(1) == 1 and b.stride(1) == 1
     K, M = (a.shape if a_mn else a.shape[::-1])
@@ -114,9 +116,10 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype, device=a.device)
     assert out.stride(1) == 1
-    rc = lib().cm_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
-                            out.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate),
-                            err_word(a.device).data_ptr(), stream_ptr())
+    args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), int(a_mn), int(b_mn),
+            int(out.dtype == torch.float32), int(accumulate))
+    err, stream = err_word(a.device).data_ptr(), stream_ptr()
+    rc = lib().cm_gemm_bf16_tiled(*args, 0, 256, err, stream) if peer_out else lib().cm_gemm_bf16(*args, err, stream)
     _check(rc, "cm_gemm_bf16")
     F_.count_launch("gemm")
     return out

@@ -202,7 +202,7 @@ class FusedTP:
             p = (me + q) % self.tp                       # remote owners first, this rank's own shard last
             dst = self.heap.peer_tensor(my_slot, p)
             for b in range(B):
-                gemm(x[b, p * Sl:(p + 1) * Sl], w, b_mn=b_mn, out=dst[b])
+                gemm(x[b, p * Sl:(p + 1) * Sl], w, b_mn=b_mn, out=dst[b], peer_out=p != me)
         self.heap.barrier(FLAG_RS, self.rs_epoch)                # every rank's partial tiles have landed here
         out = torch.empty(B, Sl, N, dtype=torch.bfloat16, device=x.device)
         rc = _lib().cm_sum_slots(stage.data_ptr(), out.data_ptr(), self.tp, n_local, stream_ptr())
