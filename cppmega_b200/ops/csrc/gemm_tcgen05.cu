@@ -487,14 +487,16 @@ static int dispatch_layout(bool a_mn, bool b_mn, const CUtensorMap& tmA, const C
 using namespace cm;
 
 // Tile shape of a dense problem.  A launch takes ceil(tiles / tiles in flight) waves; the weight of a wave is its measured time
-// (16384 x 24960 x 4096: 24.2 us with 256 columns, 20.5 with 192, 17.8 with 128; one CTA 17.9 with 128 and 14.8 with 64):
-// narrow tiles read more operand bytes per product, so they only win where they save waves.
+// (16384 x 24960 x 4096: pairs 24.2 us with 256 columns, 20.5 with 192, 17.8 with 128; one CTA 28.5 with 256, 17.9 with 128 and
+// 14.8 with 64): narrow tiles read more operand bytes per product, and half the rows cost a sixth, so they only win where they
+// save waves (300 x 24960 x 4096: 65 us in two waves of 128 x 256, 74 in three of pairs).
+// Adding to C from a short reduction is mostly epilogue, which on one CTA does not wait for a partner: with K <= 512 pairs take
+// 1.03 to 1.11 times as long (4096 x 4096 x 256 bf16: 37.2 us against 33.8), at 1024 up to 1.04, at 2048 they are ahead.
 struct DensePlan {
   int pair, bn;
 };
-static DensePlan plan_dense(int M, int N, bool b_mn) {
-  const int sms = sm_count();
-  DensePlan best{1, 256};
+static DensePlan plan_dense(int sms, int M, int N, int K, bool b_mn, bool accumulate) {
+  DensePlan best{0, 256};
   double best_cost = 1e30;
   auto consider = [&](int pair, int bn, double wave) {
     const long long tiles = (long long)((M + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((N + bn - 1) / bn);
@@ -502,12 +504,20 @@ static DensePlan plan_dense(int M, int N, bool b_mn) {
     const double cost = double((tiles + slots - 1) / slots) * wave;
     if (cost < best_cost) { best_cost = cost; best = DensePlan{pair, bn}; }
   };
-  consider(1, 256, 24.2);
-  if (!b_mn) consider(1, 192, 20.5);            // an MN-major B comes in runs of 64 columns per CTA
-  consider(1, 128, 17.8);
+  if (!(accumulate && K <= 1024)) {
+    consider(1, 256, 24.2);
+    if (!b_mn) consider(1, 192, 20.5);            // an MN-major B comes in runs of 64 columns per CTA
+    consider(1, 128, 17.8);
+  }
+  consider(0, 256, 28.5);
   consider(0, 128, 17.9);
   consider(0, 64, 14.8);
   return best;
+}
+// The choice on a chip of `sms` SMs: 1000 * pair + columns.
+extern "C" int cm_gemm_bf16_plan(int sms, int M, int N, int K, int b_mn, int accumulate) {
+  const DensePlan p = plan_dense(sms, M, N, K, b_mn != 0, accumulate != 0);
+  return 1000 * p.pair + p.bn;
 }
 
 // cm_gemm_bf16 with the tile shape given: pair = 1: bn 128 or 256, with a K-major B also 192; pair = 0: bn 64, 128 or 256.
@@ -548,7 +558,7 @@ extern "C" int cm_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
     return -10;   // TMA needs 16-byte aligned bases and row pitches
-  const DensePlan p = plan_dense(M, N, b_mn != 0);
+  const DensePlan p = plan_dense(sm_count(), M, N, K, b_mn != 0, accumulate != 0);
   return cm_gemm_bf16_tiled(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, p.pair, p.bn, err, stream);
 }
 
