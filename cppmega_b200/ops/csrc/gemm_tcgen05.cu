@@ -562,9 +562,6 @@ extern "C" int cm_gemm_bf16(const void* A, const void* B, void* C, int M, int N,
   return cm_gemm_bf16_tiled(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_fp32, accumulate, p.pair, p.bn, err, stream);
 }
 
-// Expert segments start at multiples of 128 rows, so a 256-row pair tile at a segment boundary is worked on twice.  From a
-// mean of four 128-row tiles per expert on that costs less than the pair gains; below it the one-CTA kernel stays.
-static bool pair_for_experts(int rows, int num_experts) { return rows >= num_experts * 5 * BM; }
 // Fewest column tiles, weighted by their time as in plan_dense.
 static int expert_bn(int N, bool b_mn) {
   const int n256 = (N + 255) / 256, n192 = (N + 191) / 192, n128 = (N + 127) / 128;
@@ -572,17 +569,49 @@ static int expert_bn(int N, bool b_mn) {
   return n128 * 17.8 < n256 * 24.2 ? 128 : 256;
 }
 
+// Expert segments start at multiples of 128 rows, so a 256-row pair tile that two experts share is worked on twice: half of the
+// boundaries on average, and with them the pair that has the most tiles takes one more.  Against that stands the time of a
+// wave, 0.85 of the one-CTA kernel's for reductions up to 1,024 (the epilogue is a large part), 0.93 up to 2,048, and in loops of
+// such products nothing beyond (power sets the rate).  Pair time over one-CTA time, 16 experts, hidden 4,096, ffn 896, at a mean of
+// 512 / 1,024 / 2,048 rows: w2 (K 896) 1.10 / 0.93 / 0.84, its input gradient (K 4,096) 1.70 / 1.36 / 1.02, w1 (K 4,096)
+// 1.23 / 1.22 / 1.03, its input gradient (K 1,792) 1.25 / 1.06 / 0.95.  `used_rows` are the rows routed here as the host knows
+// them; the allocated ones can be several times as many.
+static bool pair_for_experts(int sms, int used_rows, int num_experts, int N, int K, int bn) {
+  if (K > 2048) return false;
+  const int pairs = sms / 2, cols = (N + bn - 1) / bn;
+  const double tiles = used_rows / 128 + 0.5 * num_experts, row_pairs = 0.5 * tiles, passes = row_pairs + 0.5 * (num_experts - 1);
+  auto waves = [](double work, int slots) { return (long long)((work + slots - 1) / slots); };
+  const long long one = waves(tiles * ((N + 255) / 256), sms), shared = waves(passes * cols, pairs), longest = waves(row_pairs * cols, pairs) + 1;
+  const double wave = (K <= 1024 ? 0.85 : 0.93) * (bn == 256 ? 1.0 : bn == 192 ? 20.5 / 24.2 : 17.8 / 24.2);
+  return wave * double(shared > longest ? shared : longest) < double(one);
+}
+// Expert weight gradients: a pair tile needs more than one CTA's rows of C.  Added to C, a short reduction is mostly epilogue as
+// in plan_dense (mean of 16 to 768 rows: 1.00 to 1.12 of the one-CTA time, 0.96 to 1.04 at 1,024, 0.95 at 1,536); written, the
+// bulk tensor stores are ahead at any length (0.55 to 0.95).
+static bool pair_for_expert_wgrad(int used_rows, int num_experts, int M, bool accumulate) {
+  return M > BM && !(accumulate && used_rows / num_experts < 1280);
+}
+// Whether these problems run on CTA pairs on a chip of `sms` SMs.
+extern "C" int cm_grouped_rows_plan(int sms, int used_rows, int num_experts, int N, int K, int b_mn) {
+  return pair_for_experts(sms, used_rows, num_experts, N, K, expert_bn(N, b_mn != 0));
+}
+extern "C" int cm_grouped_k_plan(int used_rows, int num_experts, int M, int accumulate) {
+  return pair_for_expert_wgrad(used_rows, num_experts, M, accumulate != 0);
+}
+
 // Grouped over 128-row-aligned expert segments of A / C.
 //   b_mn = 0: C[r, :N] = A[r, :K] . W[e(r)][N,K]^T          (expert forward)
 //   b_mn = 1: C[r, :N] = A[r, :K] . W[e(r)][K,N]            (expert dgrad; W stored [E, K, N])
-// tile_expert[rows/128] gives the expert of each 128-row tile (-1: skip).
+// tile_expert[rows/128] gives the expert of each 128-row tile (-1: skip).  used_rows: the rows that carry tokens, as far as the
+// host knows; it only chooses the kernel.
 extern "C" int cm_grouped_gemm_rows_bf16(const void* A, const void* W, void* C, int rows, int N, int K, int num_experts,
-                                         int b_mn, const int* tile_expert, int* err, cudaStream_t stream) {
-  if (rows <= 0) return 0;
+                                         int b_mn, const int* tile_expert, int used_rows, int* err, cudaStream_t stream) {
+  if (rows <= 0 || num_experts <= 0) return 0;
   if (rows % BM) return -11;
   if ((K % 8) || (N % 8)) return -10;
-  if (pair_for_experts(rows, num_experts)) {
-    const PairArgs args{rows, N, K, expert_bn(N, b_mn != 0), N, num_experts, 0, 0, tile_expert, nullptr, err};
+  const int bn = expert_bn(N, b_mn != 0);
+  if (pair_for_experts(sm_count(), used_rows, num_experts, N, K, bn)) {
+    const PairArgs args{rows, N, K, bn, N, num_experts, 0, 0, tile_expert, nullptr, err};
     return launch_gemm_pair(PAIR_GROUPED_ROWS, false, b_mn, false, A, W, C, K, b_mn ? N : K, rows, args, stream);
   }
   constexpr int BN = 256;
@@ -598,13 +627,13 @@ extern "C" int cm_grouped_gemm_rows_bf16(const void* A, const void* W, void* C, 
 }
 
 // Expert weight gradients: C[e][M,N] (+)= sum over rows r in [seg[e], seg[e+1]) of A[r, :M]^T B[r, :N].
-// seg offsets are multiples of 64.  out_fp32 / accumulate as in cm_gemm_bf16.
+// seg offsets are multiples of 64.  used_rows as above, out_fp32 / accumulate as in cm_gemm_bf16.
 extern "C" int cm_grouped_gemm_k_bf16(const void* A, const void* B, void* C, int rows, int M, int N, int num_experts,
-                                      const int* seg_offsets, int out_fp32, int accumulate, int* err,
+                                      const int* seg_offsets, int used_rows, int out_fp32, int accumulate, int* err,
                                       cudaStream_t stream) {
   if (rows <= 0 || num_experts <= 0) return 0;
   if ((M % 8) || (N % 8)) return -10;
-  if (M > BM) {       // a pair tile needs more than one CTA's rows; with 128 or fewer its second half would be padding
+  if (pair_for_expert_wgrad(used_rows, num_experts, M, accumulate != 0)) {
     const PairArgs args{M, N, 0, expert_bn(N, true), N, num_experts, accumulate, 0, nullptr, seg_offsets, err};
     return launch_gemm_pair(PAIR_GROUPED_K, true, true, out_fp32, A, B, C, M, N, rows, args, stream);
   }

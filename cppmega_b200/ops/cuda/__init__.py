@@ -44,8 +44,8 @@ def _declare(L: ctypes.CDLL) -> None:
     sig = {
         "cm_gemm_bf16": [vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, i32, i32, i32, vp, vp],
         "cm_gemm_bf16_tiled": [vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, i32, i32, i32, i32, i32, vp, vp],
-        "cm_grouped_gemm_rows_bf16": [vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp],
-        "cm_grouped_gemm_k_bf16": [vp, vp, vp, i32, i32, i32, i32, vp, i32, i32, vp, vp],
+        "cm_grouped_gemm_rows_bf16": [vp, vp, vp, i32, i32, i32, i32, i32, vp, i32, vp, vp],
+        "cm_grouped_gemm_k_bf16": [vp, vp, vp, i32, i32, i32, i32, vp, i32, i32, i32, vp, vp],
         "cm_rmsnorm_fwd": [vp, vp, vp, vp, i32, i32, f32, vp],
         "cm_rmsnorm_bwd": [vp, vp, vp, vp, vp, vp, i32, i32, vp],
         "cm_swiglu_fwd": [vp, vp, i64, i32, vp],

@@ -53,19 +53,20 @@ def padded_plan(counts: torch.Tensor, total_rows: int) -> Tuple[torch.Tensor, to
 
 
 class GroupedLinearFn(torch.autograd.Function):
-    """y[r] = x[r] @ W[e(r)]^T on the padded layout; W is [E, N, K]."""
+    """y[r] = x[r] @ W[e(r)]^T on the padded layout; W is [E, N, K]; ``used_rows`` of the rows carry tokens."""
 
     @staticmethod
-    def forward(ctx, xp, w, tile_expert, seg_offsets):
+    def forward(ctx, xp, w, tile_expert, seg_offsets, used_rows):
         from . import lib, err_word, stream_ptr, _check
         rows, K = xp.shape
         E, N, _ = w.shape
         y = torch.empty(rows, N, dtype=xp.dtype, device=xp.device)
         _check(lib().cm_grouped_gemm_rows_bf16(xp.data_ptr(), w.data_ptr(), y.data_ptr(), rows, N, K, E, 0,
-                                               tile_expert.data_ptr(), err_word(xp.device).data_ptr(), stream_ptr()),
+                                               tile_expert.data_ptr(), used_rows, err_word(xp.device).data_ptr(), stream_ptr()),
                "cm_grouped_gemm_rows_bf16")
         F_.count_launch("grouped_gemm")
         ctx.save_for_backward(xp, w, tile_expert, seg_offsets)
+        ctx.used_rows = used_rows
         return y
 
     @staticmethod
@@ -81,7 +82,7 @@ class GroupedLinearFn(torch.autograd.Function):
             dx = torch.empty_like(xp)
             # reduction over N, output width K: W [E, N, K] is the "MN-major" B operand
             _check(lib().cm_grouped_gemm_rows_bf16(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), rows, K, N, E, 1,
-                                                   tile_expert.data_ptr(), err, stream_ptr()),
+                                                   tile_expert.data_ptr(), ctx.used_rows, err, stream_ptr()),
                    "cm_grouped_gemm_rows_bf16(dgrad)")
             F_.count_launch("grouped_gemm")
         if ctx.needs_input_grad[1]:
@@ -90,12 +91,12 @@ class GroupedLinearFn(torch.autograd.Function):
             def run(out, acc):
                 out = torch.empty_like(w) if out is None else out
                 _check(lib().cm_grouped_gemm_k_bf16(dy.data_ptr(), xp.data_ptr(), out.data_ptr(), rows, N, K, E,
-                                                    seg_offsets.data_ptr(), int(out.dtype == torch.float32), int(acc), err,
-                                                    stream_ptr()), "cm_grouped_gemm_k_bf16")
+                                                    seg_offsets.data_ptr(), ctx.used_rows, int(out.dtype == torch.float32), int(acc),
+                                                    err, stream_ptr()), "cm_grouped_gemm_k_bf16")
                 F_.count_launch("grouped_gemm")
                 return out
             dw = wgrad_into_main_grad(w, run)
-        return dx, dw, None, None
+        return dx, dw, None, None, None
 
 
 def moe_experts(x_sorted: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, counts: torch.Tensor):
@@ -107,9 +108,9 @@ def moe_experts(x_sorted: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, coun
     dst_row, tile_expert, seg_offsets, max_rows = padded_plan(counts, x_sorted.shape[0])
     xp = torch.zeros(max_rows, x_sorted.shape[1], dtype=x_sorted.dtype, device=x_sorted.device)
     xp = xp.index_copy(0, dst_row, x_sorted)
-    h = GroupedLinearFn.apply(xp, w1, tile_expert, seg_offsets)
+    h = GroupedLinearFn.apply(xp, w1, tile_expert, seg_offsets, x_sorted.shape[0])
     h = swiglu(h)
-    y = GroupedLinearFn.apply(h, w2, tile_expert, seg_offsets)
+    y = GroupedLinearFn.apply(h, w2, tile_expert, seg_offsets, x_sorted.shape[0])
     return y.index_select(0, dst_row)
 
 

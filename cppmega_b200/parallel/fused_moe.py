@@ -344,7 +344,7 @@ def _zero_pad(buf, plan: MoEPlan, capacity: int):
         raise RuntimeError(f"cm_moe_zero_pad_rows failed ({rc})")
 
 
-def _grouped(x, w, tile_expert, rows, b_mn, out=None):
+def _grouped(x, w, plan: MoEPlan, rows, b_mn, out=None):
     """out[r] = x[r] . W[e(r)]^T (b_mn False) or x[r] . W[e(r)] (b_mn True, W [E, red, out])."""
     from ..ops.cuda import lib, err_word, stream_ptr, _check
     E = w.shape[0]
@@ -355,13 +355,13 @@ def _grouped(x, w, tile_expert, rows, b_mn, out=None):
     if out is None:
         out = torch.empty(rows, n_out, dtype=x.dtype, device=x.device)
     _check(lib().cm_grouped_gemm_rows_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), rows, n_out, red, E, int(b_mn),
-                                           tile_expert.data_ptr(), err_word(x.device).data_ptr(), stream_ptr()),
+                                           plan.tile_expert.data_ptr(), plan.T * plan.k, err_word(x.device).data_ptr(), stream_ptr()),
            "cm_grouped_gemm_rows_bf16")
     F_.count_launch("grouped_gemm")
     return out
 
 
-def _grouped_wgrad(dy, x, seg_offsets, E, w=None):
+def _grouped_wgrad(dy, x, plan: MoEPlan, E, w=None):
     """dW[e] = dy_e^T x_e per expert segment; accumulated into ``w.main_grad`` when the optimizer allows it."""
     from ..ops.cuda import lib, err_word, stream_ptr, _check, wgrad_into_main_grad
     rows, N = dy.shape
@@ -369,8 +369,8 @@ def _grouped_wgrad(dy, x, seg_offsets, E, w=None):
 
     def run(out, acc):
         out = torch.empty(E, N, K, dtype=dy.dtype, device=dy.device) if out is None else out
-        _check(lib().cm_grouped_gemm_k_bf16(dy.data_ptr(), x.data_ptr(), out.data_ptr(), rows, N, K, E, seg_offsets.data_ptr(),
-                                            int(out.dtype == torch.float32), int(acc), err_word(dy.device).data_ptr(),
+        _check(lib().cm_grouped_gemm_k_bf16(dy.data_ptr(), x.data_ptr(), out.data_ptr(), rows, N, K, E, plan.seg_offsets.data_ptr(),
+                                            plan.T * plan.k, int(out.dtype == torch.float32), int(acc), err_word(dy.device).data_ptr(),
                                             stream_ptr()), "cm_grouped_gemm_k_bf16")
         F_.count_launch("grouped_gemm")
         return out
@@ -486,9 +486,9 @@ class _FusedMoEFn(torch.autograd.Function):
                 if fp8 is not None:
                     ch.h = _experts_fwd_mx(ch.xin, w1, w2, ch.plan.tile_expert, ch.yout, fp8 == "tensorwise")
                 else:
-                    ch.h = _grouped(ch.xin, w1, ch.plan.tile_expert, cap_c, False)
+                    ch.h = _grouped(ch.xin, w1, ch.plan, cap_c, False)
                     a = swiglu_rows(ch.h, ch.plan.seg_offsets[-1:])      # only the rows in use of the worst-case buffer
-                    _grouped(a, w2, ch.plan.tile_expert, cap_c, False, out=ch.yout)
+                    _grouped(a, w2, ch.plan, cap_c, False, out=ch.yout)
             heap.signal(ch.f0 + 1, ep0)
             ch.event = main.record_event()
         with torch.cuda.stream(comm):
@@ -546,11 +546,11 @@ class _FusedMoEFn(torch.autograd.Function):
                 else:
                     used = plan.seg_offsets[-1:]                                     # rows in use (device int32)
                     a = swiglu_rows(h, used)                                         # recompute a = swiglu(h)
-                    da = _grouped(gin[c], w2, plan.tile_expert, cap_c, True)         # [cap, F]
-                    g2 = _grouped_wgrad(gin[c], a, plan.seg_offsets, E, w2)          # [E, H, F]
+                    da = _grouped(gin[c], w2, plan, cap_c, True)                     # [cap, F]
+                    g2 = _grouped_wgrad(gin[c], a, plan, E, w2)                      # [E, H, F]
                     dh = swiglu_bwd_rows(h, da, used)
-                    _grouped(dh, w1, plan.tile_expert, cap_c, True, out=gout[c])     # [cap, H]
-                    g1 = _grouped_wgrad(dh, xin, plan.seg_offsets, E, w1)            # [E, 2F, H]
+                    _grouped(dh, w1, plan, cap_c, True, out=gout[c])                 # [cap, H]
+                    g1 = _grouped_wgrad(dh, xin, plan, E, w1)                        # [E, 2F, H]
             fused_acc = getattr(w1, "grad_added_to_main_grad", False)                # the GEMM epilogue accumulated in place
             dw1 = g1 if (dw1 is None or fused_acc) else dw1 + g1
             dw2 = g2 if (dw2 is None or getattr(w2, "grad_added_to_main_grad", False)) else dw2 + g2

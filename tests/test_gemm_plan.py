@@ -24,3 +24,43 @@ def lib():
 ])
 def test_dense_plan(lib, M, N, K, b_mn, accumulate, want):
     assert lib.cm_gemm_bf16_plan(148, M, N, K, b_mn, accumulate) == want
+
+
+@pytest.mark.parametrize("used,E,N,K,b_mn,want", [
+    (32768, 16, 4096, 896, 0, 1),               # many rows, a short reduction: pairs
+    (32768, 16, 4096, 1792, 1, 1),
+    (16384, 16, 4096, 896, 0, 1),
+    (16384, 16, 4096, 1792, 1, 0),              # shared boundary tiles cost more than the pair saves
+    (8192, 16, 4096, 896, 0, 0),
+    (32768, 16, 1792, 4096, 0, 0),              # a long reduction
+    (16384, 16, 1024, 1024, 0, 0),              # few waves
+    (32768, 16, 1024, 1024, 0, 1),
+    (64, 16, 4096, 896, 0, 0),
+])
+def test_expert_products_go_to_pairs_by_the_rows_in_use(lib, used, E, N, K, b_mn, want):
+    assert lib.cm_grouped_rows_plan(148, used, E, N, K, b_mn) == want
+
+
+@pytest.mark.parametrize("used,E,M,accumulate,want", [(64, 16, 1792, 0, 1), (64, 16, 1792, 1, 0), (20479, 16, 1792, 1, 0),
+                                                      (20480, 16, 1792, 1, 1), (65536, 16, 128, 0, 0)])
+def test_expert_weight_gradients_go_to_pairs(lib, used, E, M, accumulate, want):
+    assert lib.cm_grouped_k_plan(used, E, M, accumulate) == want
+
+
+def test_routed_experts_pass_the_rows_in_use_not_the_allocated_ones(monkeypatch):
+    """The buffers of an expert-parallel rank hold several times the rows that arrive on average."""
+    import types
+
+    import torch
+    from cppmega_b200.ops import cuda as cu
+    from cppmega_b200.parallel import fused_moe as fm
+    calls = []
+    entry = lambda *a: calls.append(a) or 0  # noqa: E731
+    monkeypatch.setattr(cu, "lib", lambda: types.SimpleNamespace(cm_grouped_gemm_rows_bf16=entry, cm_grouped_gemm_k_bf16=entry))
+    monkeypatch.setattr(cu, "err_word", lambda device=None: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(cu, "stream_ptr", lambda: 0)
+    plan = types.SimpleNamespace(T=40, k=4, tile_expert=torch.zeros(8, dtype=torch.int32), seg_offsets=torch.zeros(3, dtype=torch.int32))
+    x, w = torch.zeros(1024, 16, dtype=torch.bfloat16), torch.zeros(2, 24, 16, dtype=torch.bfloat16)
+    y = fm._grouped(x, w, plan, 1024, False)
+    fm._grouped_wgrad(y, x, plan, 2)
+    assert calls[0][9] == 160 and calls[1][8] == 160

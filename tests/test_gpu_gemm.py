@@ -138,8 +138,8 @@ def test_gemm_tile_shapes(cu, pair, bn, M, N, K, a_mn, b_mn, out, accumulate):
 
 @pytest.mark.parametrize("counts", [[700, 0, 1300, 129], [5, 640, 2000, 0], [1025, 1023, 128, 896]])
 def test_grouped_experts_pair_tiles(cu, counts):
-    """Row counts for which the expert products run on CTA pairs: segments of odd and even tile counts, empty experts, and
-    widths that end inside a tile."""
+    """Segments of odd and even tile counts, empty experts, and widths that end inside a tile, through the public entry: the
+    products of one CTA and the weight gradients of CTA pairs."""
     from cppmega_b200.ops.cuda import extra
     from cppmega_b200.ops import reference as ref
     torch.manual_seed(4)
@@ -198,3 +198,63 @@ def test_mxfp8_gemm_result_in_an_unaligned_view(cu, M, out, accumulate):
         assert ((C.double() - ref).norm() / ref.norm()).item() < (1e-5 if out == torch.float32 else 4e-3)
         C.copy_(C0)
         assert torch.equal(buf, before)
+
+
+def _expert_layout(tiles, spare):
+    """Expert segments of the given numbers of 128-row tiles, then ``spare`` unused ones: (tile_expert, seg_offsets, rows)."""
+    te = [e for e, n in enumerate(tiles) for _ in range(n)] + [-1] * spare
+    off = [0]
+    for n in tiles:
+        off.append(off[-1] + 128 * n)
+    return (torch.tensor(te, dtype=torch.int32, device="cuda"), torch.tensor(off, dtype=torch.int32, device="cuda"), 128 * len(te))
+
+
+PAIRS = 1 << 24       # rows in use that send any of these shapes to the CTA-pair kernel; the layout stays what the tensors say
+
+
+@pytest.mark.parametrize("tiles,spare", [([7, 0, 5, 1, 8, 3], 3), ([1] * 23, 0), ([0, 0, 31, 0, 2], 6), ([12, 12], 0)])
+@pytest.mark.parametrize("b_mn", [0, 1])
+@pytest.mark.parametrize("N,K", [(4104, 136), (4544, 64)])
+def test_expert_products_on_pairs_over_several_waves(cu, tiles, spare, b_mn, N, K):
+    """More than three times as many row-pair tiles as CTA pairs, so that accumulators and stages come round while tiles that two experts share are
+    worked on twice and unused ones are passed over: odd segments, empty experts first, in the middle and last."""
+    torch.manual_seed(sum(tiles) + N)
+    te, off, rows = _expert_layout(tiles, spare)
+    E = len(tiles)
+    assert cu.lib().cm_grouped_rows_plan(148, PAIRS, E, N, K, b_mn) == 1
+    x = torch.randn(rows, K, device="cuda").bfloat16()
+    x[int(off[-1]):] = float("nan")                                      # unused rows hold anything
+    w = torch.randn(E, K, N, device="cuda").bfloat16() if b_mn else torch.randn(E, N, K, device="cuda").bfloat16()
+    y = torch.full((rows, N), 3.0, device="cuda").bfloat16()
+    assert cu.lib().cm_grouped_gemm_rows_bf16(x.data_ptr(), w.data_ptr(), y.data_ptr(), rows, N, K, E, b_mn, te.data_ptr(), PAIRS,
+                                              cu.err_word(x.device).data_ptr(), cu.stream_ptr()) == 0
+    cu.check_errors()
+    for e in range(E):
+        s = slice(int(off[e]), int(off[e + 1]))
+        if s.start < s.stop:
+            ref = x[s].double() @ (w[e].double() if b_mn else w[e].double().t())
+            assert ((y[s].double() - ref).norm() / ref.norm()).item() < 4e-3, e
+    assert (y[int(off[-1]):] == 3.0).all()
+
+
+@pytest.mark.parametrize("tiles", [[3, 0, 1, 5, 0, 2, 1, 4], [0, 2, 0, 0, 1, 0, 6, 0]])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, 0), (torch.float32, 0), (torch.bfloat16, 1), (torch.float32, 1)])
+def test_expert_weight_gradients_on_pairs_over_several_waves(cu, tiles, out, accumulate):
+    """The same for the weight gradients: 240 tiles for 74 pairs, experts without rows in between (zeros, or left alone)."""
+    torch.manual_seed(len(tiles))
+    M, N, E = 1032, 1288, len(tiles)
+    _, off, rows = _expert_layout(tiles, 2)
+    assert cu.lib().cm_grouped_k_plan(PAIRS, E, M, accumulate) == 1
+    a, b = torch.randn(rows, M, device="cuda").bfloat16(), torch.randn(rows, N, device="cuda").bfloat16()
+    c = torch.randn(E, M, N, device="cuda").to(out)
+    before = c.clone()
+    assert cu.lib().cm_grouped_gemm_k_bf16(a.data_ptr(), b.data_ptr(), c.data_ptr(), rows, M, N, E, off.data_ptr(), PAIRS,
+                                           int(out == torch.float32), accumulate, cu.err_word(a.device).data_ptr(), cu.stream_ptr()) == 0
+    cu.check_errors()
+    for e in range(E):
+        s = slice(int(off[e]), int(off[e + 1]))
+        ref = a[s].double().t() @ b[s].double() + (before[e].double() if accumulate else 0)
+        if s.start == s.stop:
+            assert torch.equal(c[e].double(), ref if accumulate else torch.zeros_like(ref))
+        else:
+            assert ((c[e].double() - ref).norm() / ref.norm()).item() < (1e-5 if out == torch.float32 else 4e-3), e
