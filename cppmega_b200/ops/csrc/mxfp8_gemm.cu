@@ -614,9 +614,6 @@ extern "C" int cm_mxfp8_gemm(const void* A, const void* sfa, const void* B, cons
   if (K <= 0 || (K % 32) || (lda % 16) || (ldb % 16)) return -10;
   if ((reinterpret_cast<uintptr_t>(sfa) | reinterpret_cast<uintptr_t>(sfb) | reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15)
     return -11;
-  CUtensorMap tmA, tmB;
-  if (int rc = make_tmap_u8(&tmA, A, M, K, lda, BM)) return 100 + rc;
-  if (int rc = make_tmap_u8(&tmB, B, N, K, ldb, BN)) return 100 + rc;
   const int nkt = (K + BK - 1) / BK;
   Args args{M, N, K, ldc, (const uint8_t*)sfa, (const uint8_t*)sfb, err, nkt, nkt, nullptr, nullptr, 1, 0, 0};
   // a wave of pair tiles and a wave of one-CTA tiles cover the same area: pairs wherever they need no more waves
@@ -628,6 +625,9 @@ extern "C" int cm_mxfp8_gemm(const void* A, const void* sfa, const void* B, cons
     return accumulate ? launch_pair<float, true>(A, B, C, lda, ldb, args, pair_tiles, s)
                       : launch_pair<float, false>(A, B, C, lda, ldb, args, pair_tiles, s);
   }
+  CUtensorMap tmA, tmB;
+  if (int rc = make_tmap_u8(&tmA, A, M, K, lda, BM)) return 100 + rc;
+  if (int rc = make_tmap_u8(&tmB, B, N, K, ldb, BN)) return 100 + rc;
   if (!out_fp32) return accumulate ? launch<__nv_bfloat16, true>(tmA, tmB, C, args, s) : launch<__nv_bfloat16, false>(tmA, tmB, C, args, s);
   return accumulate ? launch<float, true>(tmA, tmB, C, args, s) : launch<float, false>(tmA, tmB, C, args, s);
 }
