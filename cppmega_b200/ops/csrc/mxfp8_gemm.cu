@@ -189,7 +189,7 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
     mbar_init(tmem_full, 1);
     mbar_init(tmem_empty, 8);
-    *abort_flag = 0;
+    *abort_flag = (args.err && *reinterpret_cast<volatile int*>(args.err) != 0) ? 1 : 0;   // an earlier kernel gave up: drain
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -197,13 +197,9 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tmem_relinquish();
   }
   tc_fence_before();
-  const bool drain = setup_barrier(args.err);
+  __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (drain) {
-    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
-    return;
-  }
 
   auto decode = [&](int tile) {
     Tile t;
@@ -247,7 +243,7 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       uint32_t stage = 0, phase = 0;
-      bool ok = true;
+      bool ok = *abort_flag == 0;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const Tile t = decode(tile);
         const uint8_t* sfa = args.sfa + ((size_t)t.mt * args.sfa_nkt + t.kt0) * 512;
@@ -271,7 +267,7 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     if (elect_one()) {
       constexpr uint32_t idesc0 = idesc_mxf8(BM, BN);
       uint32_t stage = 0, phase = 0, acc_phase = 0;
-      bool ok = true;
+      bool ok = *abort_flag == 0;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         const Tile t = decode(tile);
         if (t.nkt == 0) continue;
@@ -307,7 +303,7 @@ mxfp8_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     const int q = warp & 3;                    // TMEM lane quarter this warp may read
     const int half = (warp - 2) >> 2;          // which 128 of the 256 accumulator columns
     uint32_t acc_phase = 0;
-    bool ok = true;
+    bool ok = *abort_flag == 0;
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
       const Tile t = decode(tile);
       const int mt = t.mt, nt = t.nt;
