@@ -20,7 +20,7 @@
 // stacked [E*N, K] weights) or b_k_e columns further right (dgrad: the stacked transposed weights [N, E*K]);
 // GROUPED_K reduces over per-expert ranges of the shared K axis (token rows, multiples of 128) into a stack [E, M, N]
 // (expert weight gradients from the token-transposed operands).
-// Dense problems that fill the chip with 256-row tiles run on CTA pairs (mxfp8_pair_kernel): tcgen05.mma.cta_group::2 on a
+// Dense problems of several waves and a long reduction run on CTA pairs (mxfp8_pair_kernel): tcgen05.mma.cta_group::2 on a
 // 256 x 256 tile, each CTA with its 128 rows of A and half of B.  At 128 x 256 a CTA's shared memory takes 48 KB from TMA and
 // gives 48 KB to the tensor core per 512-cycle k tile, 192 bytes a cycle against the 128 it has; the pair needs 128.
 // The three products of an 8192 x 8192 x 4096 linear: 709 -> 560 us (2.95 PFLOP/s).
@@ -600,10 +600,22 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, void* C, const
 }  // namespace mxg
 }  // namespace cm
 
-// A [M,K] / B [N,K] E4M3 bytes (row strides lda / ldb bytes, multiples of 16); sfa / sfb swizzled scale tiles of
-// ceil(rows/128) x ceil(K/128) x 512 bytes; C [M,N] bf16 (out_fp32 = 0) or fp32, `accumulate` adds to C.
-extern "C" int cm_mxfp8_gemm(const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K, long long lda,
-                             long long ldb, long long ldc, int out_fp32, int accumulate, int* err, cudaStream_t s) {
+// Whether a dense problem runs on CTA pairs on a chip of `sms` SMs.  A wave of pair tiles covers the area of a wave of one-CTA tiles
+// and its main loop is a tenth shorter, but it starts and ends as two CTAs and its epilogue is no wider: pairs where they need
+// no more waves and the reduction is long enough.  Pair time over one-CTA time at two to fourteen waves: bf16 results K 512
+// 1.08 to 1.18, 1,024 0.96 to 1.29, 2,048 0.92 to 1.06, 4,096 0.91 to 1.00, 16,384 0.87; fp32 or added results are level at 3,072,
+// fp32 added ones at 4,096 (each moves as many bytes again).  A single wave is level at 8,192 (0.97 to 1.05; 0.88 to 0.94 at 16,384).
+extern "C" int cm_mxfp8_gemm_plan(int sms, int M, int N, int K, int out_fp32, int accumulate) {
+  using namespace cm::mxg;
+  const int tn = (N + BN - 1) / BN, pairs = sms / 2;
+  const long long pair_waves = ((long long)((M + 255) / 256) * tn + pairs - 1) / pairs, one_waves = ((long long)((M + 127) / 128) * tn + sms - 1) / sms;
+  const int min_k = one_waves == 1 ? 12288 : 2048 + 1024 * (out_fp32 != 0) + 1024 * (accumulate != 0);
+  return M > BM && pair_waves <= one_waves && K >= min_k;
+}
+
+// cm_mxfp8_gemm on CTA pairs (pair = 1) or on one CTA per tile.
+extern "C" int cm_mxfp8_gemm_tiled(const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K, long long lda,
+                                   long long ldb, long long ldc, int out_fp32, int accumulate, int pair, int* err, cudaStream_t s) {
   using namespace cm;
   using namespace cm::mxg;
   if (M <= 0 || N <= 0) return 0;
@@ -612,20 +624,27 @@ extern "C" int cm_mxfp8_gemm(const void* A, const void* sfa, const void* B, cons
     return -11;
   const int nkt = (K + BK - 1) / BK;
   Args args{M, N, K, ldc, (const uint8_t*)sfa, (const uint8_t*)sfb, err, nkt, nkt, nullptr, nullptr, 1, 0, 0};
-  // a wave of pair tiles and a wave of one-CTA tiles cover the same area: pairs wherever they need no more waves
-  const int tn = (N + BN - 1) / BN, pair_tiles = (M + 255) / 256 * tn, one_tiles = (M + 127) / 128 * tn, sms = sm_count();
-  if (M > BM && (pair_tiles + sms / 2 - 1) / (sms / 2) <= (one_tiles + sms - 1) / sms) {
+  if (pair) {
+    const int tiles = (M + 255) / 256 * ((N + BN - 1) / BN);
     if (!out_fp32)
-      return accumulate ? launch_pair<__nv_bfloat16, true>(A, B, C, lda, ldb, args, pair_tiles, s)
-                        : launch_pair<__nv_bfloat16, false>(A, B, C, lda, ldb, args, pair_tiles, s);
-    return accumulate ? launch_pair<float, true>(A, B, C, lda, ldb, args, pair_tiles, s)
-                      : launch_pair<float, false>(A, B, C, lda, ldb, args, pair_tiles, s);
+      return accumulate ? launch_pair<__nv_bfloat16, true>(A, B, C, lda, ldb, args, tiles, s)
+                        : launch_pair<__nv_bfloat16, false>(A, B, C, lda, ldb, args, tiles, s);
+    return accumulate ? launch_pair<float, true>(A, B, C, lda, ldb, args, tiles, s)
+                      : launch_pair<float, false>(A, B, C, lda, ldb, args, tiles, s);
   }
   CUtensorMap tmA, tmB;
   if (int rc = make_tmap_u8(&tmA, A, M, K, lda, BM)) return 100 + rc;
   if (int rc = make_tmap_u8(&tmB, B, N, K, ldb, BN)) return 100 + rc;
   if (!out_fp32) return accumulate ? launch<__nv_bfloat16, true>(tmA, tmB, C, args, s) : launch<__nv_bfloat16, false>(tmA, tmB, C, args, s);
   return accumulate ? launch<float, true>(tmA, tmB, C, args, s) : launch<float, false>(tmA, tmB, C, args, s);
+}
+
+// A [M,K] / B [N,K] E4M3 bytes (row strides lda / ldb bytes, multiples of 16); sfa / sfb swizzled scale tiles of
+// ceil(rows/128) x ceil(K/128) x 512 bytes; C [M,N] bf16 (out_fp32 = 0) or fp32, `accumulate` adds to C.
+extern "C" int cm_mxfp8_gemm(const void* A, const void* sfa, const void* B, const void* sfb, void* C, int M, int N, int K, long long lda,
+                             long long ldb, long long ldc, int out_fp32, int accumulate, int* err, cudaStream_t s) {
+  const int pair = cm_mxfp8_gemm_plan(cm::sm_count(), M, N, K, out_fp32, accumulate);
+  return cm_mxfp8_gemm_tiled(A, sfa, B, sfb, C, M, N, K, lda, ldb, ldc, out_fp32, accumulate, pair, err, s);
 }
 
 // Expert products on the 128-row-aligned, expert-sorted token layout.  A [rows, K] E4M3 with scales sfa; tile_expert[rows/128].

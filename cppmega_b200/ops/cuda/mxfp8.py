@@ -55,7 +55,8 @@ def _lib():
         L.cm_mxfp8_grouped_rows.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp]
         L.cm_mxfp8_grouped_k.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, vp, i32, i32, vp, vp]
         L.cm_mxfp8_gemm.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, i32, vp, vp]
-        for n in ("cm_mxfp8_quantize_rowwise", "cm_mxfp8_quantize_colwise", "cm_mxfp8_dequantize", "cm_mxfp8_swizzle_scales",
+        L.cm_mxfp8_gemm_tiled.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i32, i32, i32, vp, vp]
+        for n in ("cm_mxfp8_gemm_tiled", "cm_mxfp8_quantize_rowwise", "cm_mxfp8_quantize_colwise", "cm_mxfp8_dequantize", "cm_mxfp8_swizzle_scales",
                   "cm_mxfp8_gemm", "cm_mxfp8_quantize_both", "cm_mxfp8_grouped_rows", "cm_mxfp8_grouped_k"):
             getattr(L, n).restype = i32
         L._mx_declared = True

@@ -39,7 +39,7 @@ def _ops():
         "linear_pair": (cu.linear, [bf(4096, 512), bf(4096, 512)]),
         "linear_one_cta": (cu.linear, [bf(64, 512), bf(128, 512)]),
         "mxfp8_linear_small": (mx, [bf(96, 128), bf(96, 128)]),
-        "mxfp8_linear_large": (mx, [bf(4096, 2048), bf(4096, 2048)]),
+        "mxfp8_linear_large": (mx, [bf(4096, 4096), bf(4096, 4096)]),
         "experts": (lambda x, w1, w2: extra.moe_experts(x, w1, w2, counts), [bf(240, 128), bf(2, 128, 128), bf(2, 128, 64)]),
         "attention": (lambda q, k, v: F_.causal_attention(q, k, v, 0.1), [bf(1, 384, 2, 128), bf(1, 384, 2, 128), bf(1, 384, 2, 64)]),
         "sparse_attention": (lambda q, kv: F_.sparse_mla(q, kv, idx, 0.1, 64), [bf(1, 64, 32, 128), bf(1, 64, 128)]),

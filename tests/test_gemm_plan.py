@@ -47,6 +47,19 @@ def test_expert_weight_gradients_go_to_pairs(lib, used, E, M, accumulate, want):
     assert lib.cm_grouped_k_plan(used, E, M, accumulate) == want
 
 
+@pytest.mark.parametrize("M,N,K,fp32,accumulate,want", [
+    (8192, 4096, 8192, 0, 0, 1), (4096, 8192, 8192, 0, 0, 1),       # the products of a large projection
+    (2048, 2048, 2048, 0, 0, 0), (160, 4096, 8192, 0, 0, 0),        # a single wave
+    (2048, 2048, 16384, 0, 0, 1),
+    (4096, 4096, 1024, 0, 0, 0), (4096, 4096, 2048, 0, 0, 1),       # by the reduction and the bytes of the result
+    (4096, 4096, 2048, 1, 0, 0), (4096, 4096, 3072, 1, 0, 1), (4096, 4096, 3072, 1, 1, 0), (4096, 4096, 4096, 1, 1, 1),
+    (1056, 8192, 16384, 0, 0, 0),                                   # three waves of pairs against two
+    (128, 8192, 16384, 0, 0, 0),                                    # no second row tile
+])
+def test_mxfp8_plan(lib, M, N, K, fp32, accumulate, want):
+    assert lib.cm_mxfp8_gemm_plan(148, M, N, K, fp32, accumulate) == want
+
+
 def test_routed_experts_pass_the_rows_in_use_not_the_allocated_ones(monkeypatch):
     """The buffers of an expert-parallel rank hold several times the rows that arrive on average."""
     import types

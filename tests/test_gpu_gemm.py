@@ -180,10 +180,10 @@ def test_gemm_result_in_an_unaligned_view(cu, pair, bn, offset, pitch, out, accu
     assert torch.equal(buf, before)
 
 
-@pytest.mark.parametrize("M", [96, 288])
+@pytest.mark.parametrize("M,pair", [(96, 0), (288, 0), (288, 1)])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, True)])
-def test_mxfp8_gemm_result_in_an_unaligned_view(cu, M, out, accumulate):
-    """The same for the block-scaled GEMM, on one CTA (M <= 128) and on a CTA pair or one CTA (M > 128)."""
+def test_mxfp8_gemm_result_in_an_unaligned_view(cu, M, pair, out, accumulate):
+    """The same for the block-scaled GEMM, on one CTA and on a CTA pair."""
     from cppmega_b200.ops.cuda import mxfp8
     torch.manual_seed(M)
     N, K = 160, 96
@@ -192,7 +192,9 @@ def test_mxfp8_gemm_result_in_an_unaligned_view(cu, M, out, accumulate):
         buf = torch.randn(offset + M * pitch, device="cuda").to(out)
         before = buf.clone()
         C, C0 = (t[offset:].view(M, pitch)[:, :N] for t in (buf, before))
-        mxfp8.gemm_mxfp8(a, b, out=C, accumulate=accumulate)
+        assert mxfp8._lib().cm_mxfp8_gemm_tiled(a.payload.data_ptr(), a.swizzled().data_ptr(), b.payload.data_ptr(), b.swizzled().data_ptr(),
+                                                C.data_ptr(), M, N, K, K, K, pitch, int(out == torch.float32), int(accumulate), pair,
+                                                cu.err_word(C.device).data_ptr(), cu.stream_ptr()) == 0
         cu.check_errors()
         ref = mxfp8.dequantize(a).double() @ mxfp8.dequantize(b).double().t() + (C0.double() if accumulate else 0)
         assert ((C.double() - ref).norm() / ref.norm()).item() < (1e-5 if out == torch.float32 else 4e-3)

@@ -566,8 +566,9 @@ def test_mxfp8_quantize_both_tile_edges(rows, cols):
 
 @pytest.mark.parametrize("M,N,K", [(160, 96, 64), (256, 256, 128), (288, 416, 1056), (2080, 4128, 416), (4128, 9504, 160)])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.bfloat16, True), (torch.float32, True)])
-def test_mxfp8_gemm_pair_tiles(M, N, K, out, accumulate):
-    """Sizes that end inside the 256 x 256 x 128 tiles of the CTA-pair kernel: a missing second row tile, one scale tile of B
+@pytest.mark.parametrize("pair", [0, 1])
+def test_mxfp8_gemm_pair_tiles(M, N, K, out, accumulate, pair):
+    """Sizes that end inside the 256 x 256 x 128 tiles of the CTA-pair kernel, on it and on the one-CTA kernel: a missing second row tile, one scale tile of B
     instead of two, a last k tile of 32.  The reference multiplies the dequantised operands in 64 bits: fp32 results differ by
     the summation (below 1e-5), bf16 results by one rounding."""
     from cppmega_b200.ops import cuda as cu
@@ -577,7 +578,10 @@ def test_mxfp8_gemm_pair_tiles(M, N, K, out, accumulate):
     a = mxfp8.quantize_rowwise((torch.randn(M, K, device="cuda") * spread(M)).bfloat16())
     b = mxfp8.quantize_rowwise((torch.randn(N, K, device="cuda") * spread(N)).bfloat16())
     c0 = torch.randn(M, N, device="cuda").to(out)
-    c = mxfp8.gemm_mxfp8(a, b, out=c0.clone(), accumulate=accumulate)
+    c = c0.clone()
+    assert mxfp8._lib().cm_mxfp8_gemm_tiled(a.payload.data_ptr(), a.swizzled().data_ptr(), b.payload.data_ptr(), b.swizzled().data_ptr(),
+                                            c.data_ptr(), M, N, K, K, K, N, int(out == torch.float32), int(accumulate), pair,
+                                            cu.err_word(c.device).data_ptr(), cu.stream_ptr()) == 0
     cu.check_errors()
     # an E4M3 value times a power of two is exact in bf16
     want = mxfp8.dequantize(a).double() @ mxfp8.dequantize(b).double().t() + (c0.double() if accumulate else 0)
