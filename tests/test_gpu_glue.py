@@ -426,13 +426,14 @@ def test_moe_transport_skips_and_reports_rows_beyond_capacity():
 
 @pytest.mark.parametrize("k", [1, 3, 4, 5, 8, 9])
 @pytest.mark.parametrize("H", [8, 264, 520, 1024])
-def test_moe_pulls_over_rows_per_token_and_widths(k, H):
-    """Both pulls for row counts on either side of each kernel's limit and widths that leave a partial vector group."""
+@pytest.mark.parametrize("T", [37, 1025, 2049])
+def test_moe_pulls_over_rows_per_token_and_widths(T, k, H):
+    """Both pulls for row counts and token counts on either side of each kernel's limit and widths that leave a partial vector group."""
     from cppmega_b200.parallel import fused_moe as fm
     torch.manual_seed(k)
-    T, E = 37, 16
-    ids = torch.stack([torch.randperm(E, device="cuda")[:k] for _ in range(T)])
-    cap = 2 * E * fm.TILE
+    E = 16
+    ids = torch.rand(T, E, device="cuda").argsort(1)[:, :k].contiguous()
+    cap = (T * k // fm.TILE + 1 + E) * fm.TILE
     plan = fm.MoEPlan(ids, E, 1, 0, None, cap, None)
     heap = fm._LocalHeap()
     rows = torch.randn(cap, H, device="cuda").bfloat16()
