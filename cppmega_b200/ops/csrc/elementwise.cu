@@ -801,14 +801,15 @@ extern "C" int cm_rmsnorm_bwd(const void* x, const void* w, const void* dy, cons
   else if (H == 128) rmsnorm_bwd_small<16><<<small_grid(2), 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows);
   else if (H == 256) rmsnorm_bwd_small<32><<<small_grid(1), 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows);
   else if (H <= 32 * 1 * 8) rmsnorm_bwd_kernel<1><<<grid, 256, 0, s>>>(xp, wp, gp, rstd, dxp, dw, rows, H);
-  // rings of 32, 64 and 192 KB: 6, 3 and 1 CTAs per SM; calls of few rows take one row to a CTA
+  // rings of 32, 64 and 192 KB: 6, 3 and 1 CTAs per SM; calls of few rows take one row to a CTA.  The one CTA of a wide row has
+  // 512 threads: with 256 the row's own latency showed (16,384 x 16,384: 496 us, 469 without the ring, now 379)
   else if (H <= 128 * 1 * 8) {
     if (rows >= sm_count() * 6 * 4) return launch_rmsnorm_ring<128, 1, 2, 4>(xp, wp, gp, rstd, dxp, dw, rows, H, 6, s);
     return launch_rmsnorm_ring<128, 1, 1, 2>(xp, wp, gp, rstd, dxp, dw, rows, H, 6, s);
   } else if (H <= 256 * 2 * 8) {
     if (rows >= sm_count() * 3 * 2) return launch_rmsnorm_ring<256, 2, 2, 2>(xp, wp, gp, rstd, dxp, dw, rows, H, 3, s);
     return launch_rmsnorm_ring<256, 2, 1, 2>(xp, wp, gp, rstd, dxp, dw, rows, H, 3, s);
-  } else if (H <= 256 * 8 * 8) return launch_rmsnorm_ring<256, 8, 1, 3>(xp, wp, gp, rstd, dxp, dw, rows, H, 1, s);
+  } else if (H <= 256 * 8 * 8) return launch_rmsnorm_ring<512, 4, 1, 3>(xp, wp, gp, rstd, dxp, dw, rows, H, 1, s);
   else return -12;
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -26,7 +26,7 @@ def test_rmsnorm(rows, H):
     assert _rel(w.grad, wr.grad) < 8e-3
 
 
-@pytest.mark.parametrize("H", [264, 816, 1024, 1032, 3584, 4096, 4104])
+@pytest.mark.parametrize("H", [264, 816, 1024, 1032, 3584, 4096, 4104, 16384])
 @pytest.mark.parametrize("rows", [1, 297, 887, 889, 1187, 3553, 5003])
 def test_rmsnorm_backward_row_groups(rows, H):
     """Row counts on both sides of the thresholds at which a CTA takes two rows at a time (888 and 3552 on 148 SMs), with
