@@ -11,9 +11,6 @@
 namespace cm {
 
 constexpr int CE_THREADS = 512;
-// 16-byte vectors a thread requests before it uses the first: 4096 x 131072 took 730 us a chunk with one, 675 with four
-// (floor 325: one read and one write; the second read comes mostly from L2, and 2 x 537 M exponentials take 245)
-constexpr int CE_UNROLL = 4;
 constexpr float LOG2E = 1.4426950408889634f;
 
 __device__ __forceinline__ float ce_ex2(float x) {
@@ -27,6 +24,11 @@ __device__ __forceinline__ void ce_unpack(const uint4& v, float (&f)[8]) {
   for (int j = 0; j < 4; ++j) { const float2 t = __bfloat1622float2(b[j]); f[2 * j] = t.x; f[2 * j + 1] = t.y; }
 }
 
+// U: 16-byte vectors a thread requests before it uses the first.  With gradients 4096 x 131072 takes 491 us with four and 603 with
+// one (floor 325: one read and one write; the second read comes mostly from L2, and 2 x 537 M exponentials take 245), 4096 x 65536
+// 247 and 266; shorter rows leave most of a group empty (4096 x 8192: 59.5 us with four, 55.2 with one; 4096 x 1024: 31 and 27), and
+// without gradients it never pays (512 x 65536: 22.7 and 21.2).
+template <int U>
 __global__ void __launch_bounds__(CE_THREADS) ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ labels,
                                                                 const float* __restrict__ weights, float* __restrict__ loss_out,
                                                                 float* __restrict__ lse_out, int rows, int V, long long ld,
@@ -48,13 +50,13 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_bwd_kernel(__nv_bfloat16* _
       continue;
     }
     float mx = -INFINITY, sm = 0.f;
-    for (int i0 = threadIdx.x; i0 < nvec; i0 += CE_THREADS * CE_UNROLL) {
-      uint4 v[CE_UNROLL];
+    for (int i0 = threadIdx.x; i0 < nvec; i0 += CE_THREADS * U) {
+      uint4 v[U];
 #pragma unroll
-      for (int u = 0; u < CE_UNROLL; ++u)
+      for (int u = 0; u < U; ++u)
         if (i0 + u * CE_THREADS < nvec) v[u] = lv[i0 + u * CE_THREADS];
 #pragma unroll
-      for (int u = 0; u < CE_UNROLL; ++u) {
+      for (int u = 0; u < U; ++u) {
         if (i0 + u * CE_THREADS >= nvec) break;
         float f[8];
         ce_unpack(v[u], f);
@@ -85,13 +87,13 @@ __global__ void __launch_bounds__(CE_THREADS) ce_fwd_bwd_kernel(__nv_bfloat16* _
     if (!write_grad) continue;
     const float wgt = weights ? weights[row] : 1.f;
     const int lvec = int(label >> 3), lsub = int(label & 7);
-    for (int i0 = threadIdx.x; i0 < nvec; i0 += CE_THREADS * CE_UNROLL) {
-      uint4 v[CE_UNROLL];
+    for (int i0 = threadIdx.x; i0 < nvec; i0 += CE_THREADS * U) {
+      uint4 v[U];
 #pragma unroll
-      for (int u = 0; u < CE_UNROLL; ++u)
+      for (int u = 0; u < U; ++u)
         if (i0 + u * CE_THREADS < nvec) v[u] = lv[i0 + u * CE_THREADS];
 #pragma unroll
-      for (int u = 0; u < CE_UNROLL; ++u) {
+      for (int u = 0; u < U; ++u) {
         const int i = i0 + u * CE_THREADS;
         if (i >= nvec) break;
         float f[8];
@@ -175,7 +177,7 @@ extern "C" int cm_ce_fwd_bwd(void* logits, const long long* labels, const float*
   if (rows <= 0) return 0;
   if (V % 8 || ld % 8) return -10;
   int grid = rows < cm::sm_count() * 2 ? rows : cm::sm_count() * 2;
-  cm::ce_fwd_bwd_kernel<<<grid, cm::CE_THREADS, 0, s>>>((__nv_bfloat16*)logits, labels, weights, loss_out, lse_out, rows, V,
-                                                        ld, ignore_index, write_grad);
+  const auto kernel = write_grad && V >= 65536 ? cm::ce_fwd_bwd_kernel<4> : cm::ce_fwd_bwd_kernel<1>;
+  kernel<<<grid, cm::CE_THREADS, 0, s>>>((__nv_bfloat16*)logits, labels, weights, loss_out, lse_out, rows, V, ld, ignore_index, write_grad);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -117,10 +117,10 @@ def test_linear_ce_weighted(T, H, V):
     assert _rel(w.grad, wr.grad) < 3e-2
 
 
-@pytest.mark.parametrize("T,H,V", [(33, 64, 8), (130, 64, 16392), (4097, 64, 512)])
+@pytest.mark.parametrize("T,H,V", [(33, 64, 8), (130, 64, 16392), (70, 64, 65544), (4097, 64, 512)])
 def test_linear_ce_chunk_and_vocabulary_edges(T, H, V):
-    """A vocabulary of one vector, one that ends inside an unrolled group of vectors, and a last chunk of one row (the first
-    chunk writes dw, the second adds to it)."""
+    """A vocabulary of one vector, ones that end inside a group of vectors of either kernel, and a last chunk of one row (the
+    first chunk writes dw, the second adds to it)."""
     test_linear_ce_weighted(T, H, V)
 
 
