@@ -116,10 +116,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if out is None:
         out = torch.empty(M, N, dtype=out_dtype, device=a.device)
     assert out.stride(1) == 1
-    args = (a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0), int(a_mn), int(b_mn),
-            int(out.dtype == torch.float32), int(accumulate))
-    err, stream = err_word(a.device).data_ptr(), stream_ptr()
-    rc = lib().cm_gemm_bf16_tiled(*args, 0, 256, err, stream) if peer_out else lib().cm_gemm_bf16(*args, err, stream)
+    if peer_out:
+        rc = lib().cm_gemm_bf16_tiled(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                                      int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate), 0, 256,
+                                      err_word(a.device).data_ptr(), stream_ptr())
+    else:
+        rc = lib().cm_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0),
+                                out.stride(0), int(a_mn), int(b_mn), int(out.dtype == torch.float32), int(accumulate),
+                                err_word(a.device).data_ptr(), stream_ptr())
     _check(rc, "cm_gemm_bf16")
     F_.count_launch("gemm")
     return out

@@ -111,7 +111,7 @@ def test_linear_fp32out_router_shape():
 
 @pytest.mark.parametrize("pair,bn", [(1, 256), (1, 192), (1, 128), (0, 256), (0, 128), (0, 64)])
 @pytest.mark.parametrize("M,N,K", [(8, 8, 8), (129, 200, 72), (257, 264, 64), (520, 776, 456), (2056, 1032, 1000)])
-@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.bfloat16, True), (torch.float32, True)])
 def test_gemm_tile_shapes(cu, pair, bn, M, N, K, a_mn, b_mn, out, accumulate):
     """Every tile shape of the dense dispatch at sizes below, at and past the edges of its tiles, with a padded C pitch that
