@@ -22,8 +22,9 @@
 // (cppmega/megatron/cuda_ext/cutlass_mxfp8_gemm.cu:56-360, cuda_ext/grouped_mxfp8_gemm.cu:61-234),
 // which have no sm_100 path.
 //
-// Problems with enough 256-row tiles go to the CTA-pair kernel of gemm_pair.cu (plan_dense below); this one keeps the small
-// dense problems (128- and 64-column tiles), experts with few rows, and the peer-memory modes.
+// Problems with enough 256-row tiles go to the CTA-pair kernel of gemm_pair.cu (plan_dense and pair_for_experts below); this one
+// keeps the dense problems that fill no wave of pairs, additions to C from short reductions, experts with few rows or long
+// reductions, and the peer-memory modes.
 #include "common.cuh"
 #include "gemm_pair.cuh"
 
