@@ -52,7 +52,7 @@ struct PairArgs {
   long long ldc;
   int num_experts;
   int accumulate;          // C += result
-  int tma_store;           // C tiles leave through shared memory and a bulk tensor store (16-byte aligned C and pitch)
+  int tma_store;           // C tiles leave through shared memory and a bulk tensor store (C, pitch and width multiples of 16 bytes)
   const int* tile_expert;
   const int* seg_offsets;
   int* err;

@@ -180,6 +180,24 @@ def test_gemm_result_in_an_unaligned_view(cu, pair, bn, offset, pitch, out, accu
     assert torch.equal(buf, before)
 
 
+@pytest.mark.parametrize("pair,bn", [(1, 256), (1, 192), (1, 128), (0, 256), (0, 128), (0, 64)])
+@pytest.mark.parametrize("M,N,K,pitch", [(129, 201, 73, 208), (300, 515, 64, 520), (64, 1, 64, 8), (257, 66, 200, 72), (40, 260, 64, 264)])
+@pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.float32, True)])
+def test_gemm_result_of_an_odd_width_in_wider_rows(cu, pair, bn, M, N, K, pitch, out, accumulate):
+    """Rows that end off a 16-byte boundary inside aligned wider ones (out=buf[:, :N]): the columns beside them stay."""
+    torch.manual_seed(N)
+    ld = (K + 7) // 8 * 8
+    a, b = torch.randn(M, ld, device="cuda").bfloat16(), torch.randn(N, ld, device="cuda").bfloat16()
+    buf = torch.randn(M, pitch, device="cuda").to(out)
+    before = buf.clone()
+    assert cu.lib().cm_gemm_bf16_tiled(a.data_ptr(), b.data_ptr(), buf.data_ptr(), M, N, K, ld, ld, pitch, 0, 0, int(out == torch.float32),
+                                       int(accumulate), pair, bn, cu.err_word(a.device).data_ptr(), cu.stream_ptr()) == 0
+    cu.check_errors()
+    ref = a[:, :K].double() @ b[:, :K].double().t() + (before[:, :N].double() if accumulate else 0)
+    assert ((buf[:, :N].double() - ref).norm() / ref.norm()).item() < (1e-5 if out == torch.float32 else 4e-3)
+    assert torch.equal(buf[:, N:], before[:, N:])
+
+
 @pytest.mark.parametrize("M,pair", [(96, 0), (288, 0), (288, 1)])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, True)])
 def test_mxfp8_gemm_result_in_an_unaligned_view(cu, M, pair, out, accumulate):
