@@ -426,7 +426,8 @@ int launch_gemm_pair(int mode, bool a_mn, bool b_mn, bool out_fp32, const void* 
   const int es = out_fp32 ? 4 : 2;
   const bool c_aligned = (reinterpret_cast<uintptr_t>(C) & 15) == 0;
   // a bulk store cuts a row off at the next multiple of 16 bytes, not at its last element: rows that end elsewhere go element-wise
-  args.tma_store = !args.accumulate && c_aligned && (args.ldc * es) % 16 == 0 && ((long long)args.N * es) % 16 == 0;
+  args.tma_store = !args.accumulate && c_aligned && (args.ldc * es) % 16 == 0 && ((long long)args.N * es) % 16 == 0 &&
+                   args.ldc >= args.N;     // a single row may come with any pitch, which a tensor map does not take
   args.c_vec = c_aligned && args.ldc % 8 == 0;
   if (args.tma_store) {
     rc = pair2::make_store_map(&tmC, C, out_fp32, mode == PAIR_GROUPED_K, args);

@@ -198,6 +198,20 @@ def test_gemm_result_of_an_odd_width_in_wider_rows(cu, pair, bn, M, N, K, pitch,
     assert torch.equal(buf[:, N:], before[:, N:])
 
 
+@pytest.mark.parametrize("ldc", [0, 8, 64])
+def test_gemm_single_row_of_any_pitch(cu, ldc):
+    """The pitch of a single row is any number (an expanded or reshaped [1, N] view)."""
+    torch.manual_seed(ldc)
+    a, b = torch.randn(1, 64, device="cuda").bfloat16(), torch.randn(512, 64, device="cuda").bfloat16()
+    out = torch.empty(512, device="cuda").bfloat16()
+    for pair, bn in ((1, 256), (1, 128), (0, 256), (0, 64)):
+        out.zero_()
+        assert cu.lib().cm_gemm_bf16_tiled(a.data_ptr(), b.data_ptr(), out.data_ptr(), 1, 512, 64, 64, 64, ldc, 0, 0, 0, 0, pair, bn,
+                                           cu.err_word(a.device).data_ptr(), cu.stream_ptr()) == 0, (pair, bn)
+        cu.check_errors()
+        assert _rel(out, (a.float() @ b.float().t())[0]) < 4e-3
+
+
 @pytest.mark.parametrize("M,pair", [(96, 0), (288, 0), (288, 1)])
 @pytest.mark.parametrize("out,accumulate", [(torch.bfloat16, False), (torch.float32, True)])
 def test_mxfp8_gemm_result_in_an_unaligned_view(cu, M, pair, out, accumulate):
