@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) quantize_colwise_kernel(const __nv_bfloat
 // of one 32-row block, so a bank word is one read.  A tile is one line (128 bytes) of every row and of every transposed row,
 // and exactly one 128x4 scale tile of each orientation, which leaves as whole words.  Memory-bound; with 32 x 256 tiles of
 // fp32 in shared memory, 32-byte transposed runs and log2 / exp2 per block, 8192 x 8192
-// and 8192 x 4096 together took 201 us; now 104 to 137 by box.
+// and 8192 x 4096 together took 201 us; now 104 to 137.
 constexpr int QB_LD = 65;                                   // words per row of 128 bf16; each 32-row block is 8 words further
 __device__ __forceinline__ int qb_word(int row, int pair) { return row * QB_LD + (row >> 5) * 8 + pair; }
 
